@@ -4,6 +4,7 @@ import os
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "lib", "liblitert_b200.so")
+HOST_OPS_PATH = os.path.join(_HERE, "lib", "_host_ops.so")
 
 _vp = ctypes.c_void_p
 _i = ctypes.c_int
@@ -131,6 +132,23 @@ def load():
             fn.argtypes = args
         _lib = lib
     return _lib
+
+
+class _Missing:
+    def __getattr__(self, name):
+        raise B200Error(f"{HOST_OPS_PATH} is missing: build it with `python -m litert_b200.build`")
+
+
+def host_ops():
+    """The native form of the small calls (csrc/host_ops.cc); a call raises where it is not built."""
+    if not os.path.exists(HOST_OPS_PATH):
+        return _Missing()
+    import importlib.util
+    load()
+    spec = importlib.util.spec_from_file_location("_host_ops", HOST_OPS_PATH)
+    module = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(module)
+    return module
 
 
 def check(rc):

@@ -57,8 +57,30 @@ def build_kernels(force=False, verbose=False):
     return out
 
 
+def build_host_ops(force=False):
+    """The CPython extension of the small calls (csrc/host_ops.cc), over the kernels' library and torch's C++ API."""
+    import sysconfig
+
+    import torch
+
+    kernels = build_kernels()
+    out = os.path.join(LIB, "_host_ops.so")
+    src = os.path.join(CSRC, "host_ops.cc")
+    if not force and not _newer(out, [src, os.path.join(os.path.dirname(HERE), "include", "litert_b200.h")]):
+        return out
+    root = os.path.dirname(torch.__file__)
+    inc = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+           sysconfig.get_paths()["include"], os.path.join(os.path.dirname(os.path.dirname(NVCC)), "include")]
+    subprocess.check_call(["g++", "-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-shared", "-o", out, src,
+                           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"] +
+                          [f for d in inc for f in ("-isystem", d)] +
+                          ["-L" + LIB, "-l:" + os.path.basename(kernels), "-Wl,-rpath,$ORIGIN", "-L" + os.path.join(root, "lib"),
+                           "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-lc10_cuda", "-lc10"])
+    return out
+
+
 def build_all(force=False, verbose=False):
-    paths = [build_kernels(force, verbose)]
+    paths = [build_kernels(force, verbose), build_host_ops(force)]
     try:
         from . import build_delegate
     except ImportError:

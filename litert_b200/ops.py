@@ -13,6 +13,8 @@ import torch
 from . import _lib
 from ._lib import B200Error, check
 
+_host = _lib.host_ops()
+
 ACT_NONE, ACT_RELU, ACT_RELU_N1_TO_1, ACT_RELU6, ACT_TANH, ACT_SIGN_BIT, ACT_SIGMOID = range(7)
 DTYPE_F16, DTYPE_I8, DTYPE_F32 = 0, 1, 2
 
@@ -112,6 +114,10 @@ def fully_connected_int8(x, weights, bias, input_zero_point, output_zero_point, 
                          act_max=127, filter_zero_point=0, ws=None, out=None):
     """Full-integer FULLY_CONNECTED (tflite/kernels/fully_connected.cc:1383-1421 per channel, 1255-1285 per
     tensor). x int8 [..., k]; multipliers/shifts int32 tensors with n entries (per channel) or one."""
+    y = _host.fc_int8(x, weights, bias, -input_zero_point, -filter_zero_point, output_zero_point, multipliers, shifts,
+                      act_min, act_max, ws, out)
+    if y is not None:
+        return y
     lib = _lib.load()
     x = _need(x, torch.int8, "x")
     k = weights.k
@@ -133,6 +139,9 @@ def fully_connected_int8(x, weights, bias, input_zero_point, output_zero_point, 
 def fully_connected_hybrid(x, weights, filter_scales, bias=None, asymmetric_quantize_inputs=True,
                            activation=ACT_NONE, ws=None, out=None):
     """Dynamic-range FULLY_CONNECTED, EvalHybridDense (tflite/kernels/fully_connected.cc:763-858)."""
+    y = _host.fc_hybrid(x, weights, filter_scales, bias, asymmetric_quantize_inputs, activation, ws, out)
+    if y is not None:
+        return y
     lib = _lib.load()
     x = _need(x, torch.float32, "x")
     k = weights.k
@@ -152,6 +161,9 @@ def fully_connected_hybrid(x, weights, filter_scales, bias=None, asymmetric_quan
 
 def fully_connected_blockwise4(x, weights, bias=None, ws=None, out=None):
     """Blockwise int4 FULLY_CONNECTED, EvalBlockwise4Bit (tflite/kernels/fully_connected.cc:1014-1086)."""
+    y = _host.fc_w4(x, weights, bias, ws, out)
+    if y is not None:
+        return y
     lib = _lib.load()
     x = _need(x, torch.float32, "x")
     k = weights.k
@@ -171,6 +183,9 @@ _DT = {torch.float16: DTYPE_F16, torch.int8: DTYPE_I8, torch.float32: DTYPE_F32}
 def sdpa_decode(q, k, v, lengths=None, mask=None, scale=None, logit_cap=0.0, k_scale=None, v_scale=None, ws=None):
     """odml.scaled_dot_product_attention for one query token per sequence
     (tflite/experimental/genai/sdpa.cc:361-662). q [b,1,n,h]; k, v [b,s_max,nkv,h]."""
+    y = _host.sdpa_decode(q, k, v, lengths, mask, scale, logit_cap, k_scale, v_scale, ws)
+    if y is not None:
+        return y
     lib = _lib.load()
     if q.dtype not in (torch.float16, torch.float32) or k.dtype not in _DT or v.dtype != k.dtype:
         raise B200Error("unsupported dtypes for sdpa_decode")
