@@ -193,5 +193,10 @@ bool attn_step_supported(int n, int nkv, int h, int kv_dtype);
 cudaError_t launch_attn_step(const AttnStepParams& p, cudaStream_t s);
 cudaError_t launch_sdpa_decode(const SdpaParams& p, cudaStream_t s);
 size_t sdpa_workspace_bytes(int b, int n, int nkv, int h, int s_max, int shared_kv = 0);
+size_t sdpa_chunk_workspace_bytes(int b, int nkv, int h, int s_max, int shared_kv = 0);
+// One query row per sequence (sdpa_split.cu): the ragged decode step.
+bool sdpa_split_supported(const SdpaParams& p);
+cudaError_t launch_sdpa_split(const SdpaParams& p, cudaStream_t s);
+size_t sdpa_split_workspace_bytes(int b, int nkv, int h, int s_max);
 
 }  // namespace b200

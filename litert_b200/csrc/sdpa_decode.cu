@@ -1,6 +1,5 @@
-// Flash-decode for odml.scaled_dot_product_attention with one query token per
-// sequence: ragged key/value lengths, grouped-query heads, fp16 / int8 / fp32
-// key-value caches, optional additive mask and logit cap.
+// Attention over a key-value cache: the rows of a prompt pass, a decoder layer's whole attention step in one launch,
+// and the fallback for head layouts that nothing else takes (the ragged decode step is in sdpa_split.cu).
 //
 // Math (tflite/experimental/genai/sdpa.cc:361-662): for each query head n of
 // batch entry b, out = softmax_s(scale * q.k_s + mask_s) . v_s over the first
@@ -21,6 +20,8 @@
 //    softmax state; warps merge in shared memory, CTAs through a small
 //    workspace that a second kernel reduces.
 #include <math_constants.h>
+
+#include <algorithm>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -355,79 +356,8 @@ struct WarpAttention {
   }
 };
 
-template <int KV, int H, bool QF32, int GPI>
-__global__ void __launch_bounds__(kWarps * 32) sdpa_decode_kernel(const SdpaParams p, const int chunk_tokens,
-                                                                  const int chunks_max) {
-  using WA = WarpAttention<KV, H, GPI>;
-  constexpr int KSTEPS = WA::KSTEPS;
-  pdl_enter();
-  const int b = blockIdx.z, kvh = blockIdx.y, chunk = blockIdx.x;
-  const int len = p.lengths ? max(0, min(p.lengths[b], p.s_max)) : p.s_max;
-  const int c0 = chunk * chunk_tokens;
-  if (c0 >= len) return;
-  const int c1 = min(len, c0 + chunk_tokens);
-
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int g = lane >> 2, t = lane & 3;
-  const int group = p.n / p.nkv;  // query heads per kv head (<= 8)
-
-  // ---- Q fragments: thread (g,t) keeps head g, 16-byte pieces t + 4 i ----
-  uint32_t qf[KSTEPS][4];
-  {
-    const bool head_ok = g < group;
-    const int head = kvh * group + (head_ok ? g : 0);
-#pragma unroll
-    for (int i = 0; i < KSTEPS; ++i) {
-      const int d0 = 8 * (t + 4 * i);
-      if (!head_ok) {
-        qf[i][0] = qf[i][1] = qf[i][2] = qf[i][3] = 0u;
-      } else if constexpr (QF32) {
-        const float* q = static_cast<const float*>(p.q) + ((size_t)b * p.n + head) * H + d0;
-        load8<kKvF32>(q, 0, true, qf[i]);
-      } else {
-        const __half* q = static_cast<const __half*>(p.q) + ((size_t)b * p.n + head) * H + d0;
-        load8<kKvF16>(q, 0, true, qf[i]);
-      }
-    }
-  }
-  WA wa;
-  wa.template run<kSrcGlobal>(p, qf, WA::cache_rows(p, b, kvh), b, c0 + warp * WA::kTokensPerWarpIter, kWarps * WA::kTokensPerWarpIter, c1, lane);
-
-  // ---- merge the warps of this CTA ----
-  __shared__ float sm_m[kWarps][8], sm_l[kWarps][8];
-  __shared__ float sm_o[kWarps][8][H + 4];
-  wa.park(sm_m, sm_l, sm_o, warp, lane);
-  __syncthreads();
-  float* part = p.ws + ((((size_t)b * p.nkv + kvh) * chunks_max + chunk) * 8) * partial_stride(H);
-  for (int idx = tid; idx < group * H; idx += kWarps * 32) {
-    const int head = idx / H, d = idx % H;
-    float mm = -CUDART_INF_F;
-#pragma unroll
-    for (int w = 0; w < kWarps; ++w) mm = fmaxf(mm, sm_m[w][head]);
-    const float muse = mm == -CUDART_INF_F ? 0.0f : mm;
-    float acc = 0.0f, l = 0.0f;
-#pragma unroll
-    for (int w = 0; w < kWarps; ++w) {
-      const float f = exp2f(sm_m[w][head] - muse);
-      acc += f * sm_o[w][head][d];
-      l += f * sm_l[w][head];
-    }
-    float* rec = part + (size_t)head * partial_stride(H);
-    rec[d] = acc;
-    if (d == 0) {
-      rec[H] = mm;
-      rec[H + 1] = l;
-    }
-  }
-}
-
-// Staged variant of the kernel above for fp16 / int8 caches: the CTA's chunk goes through a ring of
-// shared-memory stages of kRingTokens tokens, every cached row fetched by one bulk asynchronous copy
-// (one row per thread and stage: keys by the lower half of the CTA, values by the upper), so a
-// CTA keeps up to stages x 64 KB in flight without holding registers for it, and the warps read
-// their MMA fragments from shared memory (the loads straight from global memory of the kernel
-// above leave the SMs waiting on the long scoreboard with ~7 warps each). Same chunking, same
-// partial records.
+// Ring of shared-memory stages of kRingTokens tokens: every cached row fetched by one bulk asynchronous copy
+// (one row per thread and stage: keys by the lower half of the CTA, values by the upper).
 constexpr int kRingTokens = 64;
 constexpr int kRingStagesMax = 3;
 
@@ -442,149 +372,6 @@ struct RingLayout {
     return (ring > (size_t)kParkBytes ? ring : (size_t)kParkBytes) + 128;
   }
 };
-
-template <int KV, int H, bool QF32>
-__global__ void __launch_bounds__(kWarps * 32) sdpa_decode_ring_kernel(const SdpaParams p, const int chunk_tokens,
-                                                                       const int chunks_max, const int stages,
-                                                                       const int stage_tokens) {
-  using WA = WarpAttention<KV, H, 1>;
-  using L = RingLayout<KV, H>;
-  constexpr int KSTEPS = WA::KSTEPS;
-  static_assert(kWarps * 32 == 2 * kRingTokens, "one row copy per thread and stage");
-  static_assert(kWarps * 16 == kRingTokens, "one 16-token group per warp and stage");
-  // `stage_tokens` (a multiple of 16, at most kRingTokens) tokens per stage: two stages must fit beside a
-  // second CTA on the SM, so that the copy of the next stage runs under the arithmetic of this one
-  const int stage_bytes = 2 * stage_tokens * L::kPitch;
-  extern __shared__ __align__(128) uint8_t ring_smem[];
-  __shared__ float sm_m[kWarps][8], sm_l[kWarps][8];
-  __shared__ int s_abort;
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(ring_smem);  // [kRingStagesMax], 128 bytes reserved
-  uint8_t* ring = ring_smem + 128;
-  float (*sm_o)[8][H + 4] = reinterpret_cast<float (*)[8][H + 4]>(ring);  // after the loop
-  volatile int* abort_flag = &s_abort;
-
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (tid == 0) {
-    for (int i = 0; i < kRingStagesMax; ++i) mbar_init(&full_bar[i], 1);
-    s_abort = 0;
-    mbar_fence_init();
-  }
-  pdl_enter();
-  __syncthreads();
-  const int b = blockIdx.z, kvh = blockIdx.y, chunk = blockIdx.x;
-  const int len = p.lengths ? max(0, min(p.lengths[b], p.s_max)) : p.s_max;
-  const int c0 = chunk * chunk_tokens;
-  if (c0 >= len) return;  // uniform over the CTA, nothing in flight
-  const int c1 = min(len, c0 + chunk_tokens);
-  const int n_sub = (c1 - c0 + stage_tokens - 1) / stage_tokens;
-  const int g = lane >> 2, t = lane & 3;
-  const int group = p.n / p.nkv;
-  const typename WA::Rows cache = WA::cache_rows(p, b, kvh);
-  // With one kv head the cached rows of consecutive tokens follow one another in memory: a stage is then
-  // ONE bulk copy per operand (32 KB of fp16 rows) instead of one per row, unpadded in shared memory. (128
-  // copies of 512 bytes per stage keep the copy engine busier issuing than moving; the 2- to 4-way bank
-  // conflicts of the unpadded rows cost the fragment loads less than that.)
-  const bool contiguous = cache.stride == (size_t)L::kRowBytes;
-  const int pitch = contiguous ? L::kRowBytes : L::kPitch;
-
-  // stage `s` <- tokens [c0 + j * 64, ...): thread r (< 64) fetches key row r, thread 64 + r value row r
-  auto issue = [&](int j) {
-    const int s = j % stages;
-    const int t0 = c0 + j * stage_tokens;
-    const int rows = min(stage_tokens, c1 - t0);
-    uint8_t* stage = ring + (size_t)s * stage_bytes;
-    if (tid == 0) mbar_arrive_expect_tx(&full_bar[s], (uint32_t)(2 * rows * L::kRowBytes));
-    if (contiguous) {
-      if (tid == 0) {
-        bulk_g2s(stage, cache.k + (size_t)t0 * cache.stride, (uint32_t)(rows * L::kRowBytes), &full_bar[s]);
-        bulk_g2s(stage + (size_t)stage_tokens * L::kPitch, cache.v + (size_t)t0 * cache.stride, (uint32_t)(rows * L::kRowBytes),
-                 &full_bar[s]);
-      }
-      return;
-    }
-    const int r = tid & (kRingTokens - 1);
-    if (r < rows) {
-      const bool is_v = tid >= kRingTokens;
-      const uint8_t* src = (is_v ? cache.v : cache.k) + (size_t)(t0 + r) * cache.stride;
-      bulk_g2s(stage + (size_t)(is_v ? stage_tokens : 0) * L::kPitch + (size_t)r * L::kPitch, src, L::kRowBytes, &full_bar[s]);
-    }
-  };
-  int issued = min(stages, n_sub);
-  for (int j = 0; j < issued; ++j) issue(j);
-
-  // ---- Q fragments (as above) while the first stages land ----
-  uint32_t qf[KSTEPS][4];
-  {
-    const bool head_ok = g < group;
-    const int head = kvh * group + (head_ok ? g : 0);
-#pragma unroll
-    for (int i = 0; i < KSTEPS; ++i) {
-      const int d0 = 8 * (t + 4 * i);
-      if (!head_ok) {
-        qf[i][0] = qf[i][1] = qf[i][2] = qf[i][3] = 0u;
-      } else if constexpr (QF32) {
-        const float* q = static_cast<const float*>(p.q) + ((size_t)b * p.n + head) * H + d0;
-        load8<kKvF32>(q, 0, true, qf[i]);
-      } else {
-        const __half* q = static_cast<const __half*>(p.q) + ((size_t)b * p.n + head) * H + d0;
-        load8<kKvF16>(q, 0, true, qf[i]);
-      }
-    }
-  }
-  WA wa;
-  wa.clear();
-  for (int j = 0; j < n_sub; ++j) {
-    const int s = j % stages;
-    mbar_wait_bounded(&full_bar[s], (uint32_t)(j / stages) & 1u, abort_flag, p.status, kStatusWaitTimeoutFull);
-    const int t0 = c0 + j * stage_tokens;
-    const int t1 = min(c1, t0 + stage_tokens);
-    const int first = t0 + warp * 16;
-    if (first < t1 && !*abort_flag) {
-      typename WA::Rows rows = cache;  // scales stay in global memory
-      const uint8_t* stage = ring + (size_t)s * stage_bytes;
-      rows.k = stage - (ptrdiff_t)t0 * pitch;  // indexed by absolute token
-      rows.v = stage + (size_t)stage_tokens * L::kPitch - (ptrdiff_t)t0 * pitch;
-      rows.stride = pitch;
-      wa.template run<kSrcShared>(p, qf, rows, b, first, kRingTokens, t1, lane, /*fresh=*/false, /*finish=*/false);
-    }
-    __syncthreads();  // every warp is done with stage s
-    if (issued < n_sub && !*abort_flag) {  // (abort_flag cannot change between the barrier above and here)
-      issue(issued);
-      ++issued;
-    }
-  }
-  wa.finish_sums();
-  // after an abort: the latest copies towards each stage may still be in flight
-  if (*abort_flag)
-    for (int j = max(0, issued - stages); j < issued; ++j)
-      mbar_drain_bounded(&full_bar[j % stages], (uint32_t)(j / stages) & 1u);
-  __syncthreads();
-
-  // ---- merge the warps of this CTA (the parked outputs reuse the ring) ----
-  wa.park(sm_m, sm_l, sm_o, warp, lane);
-  __syncthreads();
-  float* part = p.ws + ((((size_t)b * p.nkv + kvh) * chunks_max + chunk) * 8) * partial_stride(H);
-  for (int idx = tid; idx < group * H; idx += kWarps * 32) {
-    const int head = idx / H, d = idx % H;
-    float mm = -CUDART_INF_F;
-#pragma unroll
-    for (int w = 0; w < kWarps; ++w) mm = fmaxf(mm, sm_m[w][head]);
-    const float muse = mm == -CUDART_INF_F ? 0.0f : mm;
-    float acc = 0.0f, l = 0.0f;
-#pragma unroll
-    for (int w = 0; w < kWarps; ++w) {
-      const float f = exp2f(sm_m[w][head] - muse);
-      acc += f * sm_o[w][head][d];
-      l += f * sm_l[w][head];
-    }
-    float* rec = part + (size_t)head * partial_stride(H);
-    rec[d] = acc;
-    if (d == 0) {
-      rec[H] = mm;
-      rec[H + 1] = l;
-    }
-  }
-}
 
 // Prompt-pass variant (SdpaParams::shared_kv): the rows of the batch are consecutive tokens of ONE
 // sequence and all read the same cache, row b up to lengths[b]. Here a WARP owns a row: the warps of a
@@ -1389,10 +1176,9 @@ int pick_chunk_tokens(int b, int s_max, int shared_kv) {
 }
 
 template <int KV, int H, bool QF32>
-cudaError_t launch_fast(const SdpaParams& p, cudaStream_t s) {
+cudaError_t launch_rows(const SdpaParams& p, cudaStream_t s) {
   const int chunk_tokens = pick_chunk_tokens(p.b, p.s_max, p.shared_kv);
   const int chunks_max = (p.s_max + chunk_tokens - 1) / chunk_tokens;
-  dim3 grid(chunks_max, p.nkv, p.b);
   cudaError_t e;
   bool staged = false;
   static const bool ring_env = [] {  // B200_SDPA_RING=0: measurement knob, keeps the register-fed kernel
@@ -1401,51 +1187,7 @@ cudaError_t launch_fast(const SdpaParams& p, cudaStream_t s) {
   }();
   if constexpr (KV != kKvF32) {
     const bool aligned = ((reinterpret_cast<uintptr_t>(p.k) | reinterpret_cast<uintptr_t>(p.v)) & 15) == 0;
-    if (ring_env && !p.shared_kv && aligned && chunk_tokens % kRingTokens == 0) {
-      using L = RingLayout<KV, H>;
-      // As many stages as keep two or three CTAs on an SM: the token loop is latency-bound and wants
-      // warps more than it wants depth. Measured on B200, 16 ragged sequences up to 8192 tokens, head
-      // size 256: fp16 rows (68 KB per stage) 23.4 us with one stage, 31.4 with three (one CTA per
-      // SM); int8 rows (35 KB) 18.4 us with three, 21.9 with one. The register-fed kernel: 24.8 / 68 us.
-      // Two CTAs per SM (about 104 KB each), at least two stages per CTA so that the next stage's copy runs
-      // under this stage's arithmetic: with ONE 64-token stage per CTA (three CTAs per SM) every CTA of the
-      // grid loads, computes, loads ... in step with the others, HBM idle half of the time (device-timer
-      // stamps of one CTA, 16 ragged sequences, fp16 rows: 2.0 us copy + 1.8 us arithmetic per stage, strictly
-      // in turn). Rows that do not fit two 64-token stages get shorter stages (fp16 at head size 256: 48).
-      int stage_tokens = kRingTokens;
-      while (stage_tokens > 16 && 2 * (2 * stage_tokens * L::kPitch) > 104 * 1024) stage_tokens -= 16;
-      const int stage_bytes = 2 * stage_tokens * L::kPitch;
-      int stages = std::min(kRingStagesMax, (chunk_tokens + stage_tokens - 1) / stage_tokens);
-      stages = std::min(stages, std::max(1, (104 * 1024) / stage_bytes));
-      static const int stages_env = [] {  // B200_SDPA_STAGES: measurement knob
-        const char* e = tuning_env("B200_SDPA_STAGES");
-        return e ? atoi(e) : 0;
-      }();
-      if (stages_env >= 1 && stages_env <= kRingStagesMax) stages = std::min(stages, stages_env);
-      static const int tokens_env = [] {  // B200_SDPA_STAGE_TOKENS: measurement knob
-        const char* e = tuning_env("B200_SDPA_STAGE_TOKENS");
-        return e ? atoi(e) : 0;
-      }();
-      if (tokens_env == 16 || tokens_env == 32 || tokens_env == 48 || tokens_env == 64) stage_tokens = tokens_env;
-      const size_t ring_bytes = (size_t)stages * (2 * stage_tokens * L::kPitch);
-      const size_t smem = (ring_bytes > (size_t)L::kParkBytes ? ring_bytes : (size_t)L::kParkBytes) + 128;
-      auto kernel = sdpa_decode_ring_kernel<KV, H, QF32>;
-      static size_t configured[64] = {0};
-      int dev = 0;
-      cudaGetDevice(&dev);
-      if (dev < 0 || dev >= 64) dev = 0;
-      if (configured[dev] < smem) {
-        cudaError_t ea = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::smem_bytes(kRingStagesMax));
-        if (ea != cudaSuccess) return ea;
-        configured[dev] = L::smem_bytes(kRingStagesMax);
-      }
-      e = launch_chained(kernel, grid, dim3(kWarps * 32), smem, s, p, chunk_tokens, chunks_max, stages, stage_tokens);
-      staged = true;
-    }
-  }
-  if constexpr (KV != kKvF32) {
-    const bool aligned = ((reinterpret_cast<uintptr_t>(p.k) | reinterpret_cast<uintptr_t>(p.v)) & 15) == 0;
-    if (ring_env && p.shared_kv && aligned && chunk_tokens % kRingTokens == 0) {
+    if (ring_env && aligned && chunk_tokens % kRingTokens == 0) {
       using L = RingLayout<KV, H>;
       // Whole 64-token stages here, even when only one fits: a warp's pass covers 64 tokens, and this kernel
       // is bound by its arithmetic, not by the copies (1024-token prompt, fp16 rows, measured per layer:
@@ -1478,7 +1220,7 @@ cudaError_t launch_fast(const SdpaParams& p, cudaStream_t s) {
   }
   if (staged) {
     // (the merge below is common to all variants)
-  } else if (p.shared_kv) {
+  } else {
     // prompt pass: a warp per row, the CTA's rows share the chunk's traffic; long passes
     const dim3 rgrid(chunks_max, p.nkv, (p.b + kWarps - 1) / kWarps);
     static const int gpi = [] {  // B200_ROWS_GPI: measurement knob
@@ -1492,12 +1234,6 @@ cudaError_t launch_fast(const SdpaParams& p, cudaStream_t s) {
     } else {
       e = launch_chained(sdpa_rows_kernel<KV, H, QF32, 2>, rgrid, dim3(kWarps * 32), 0, s, p, chunk_tokens, chunks_max);
     }
-  } else if (chunk_tokens == 64) {
-    e = launch_chained(sdpa_decode_kernel<KV, H, QF32, 1>, grid, dim3(kWarps * 32), 0, s, p, chunk_tokens, chunks_max);
-  } else if (chunk_tokens == 128) {
-    e = launch_chained(sdpa_decode_kernel<KV, H, QF32, 2>, grid, dim3(kWarps * 32), 0, s, p, chunk_tokens, chunks_max);
-  } else {
-    e = launch_chained(sdpa_decode_kernel<KV, H, QF32, 4>, grid, dim3(kWarps * 32), 0, s, p, chunk_tokens, chunks_max);
   }
   if (e != cudaSuccess) return e;
   if (p.q_tiled_out) {
@@ -1517,13 +1253,13 @@ cudaError_t launch_fast(const SdpaParams& p, cudaStream_t s) {
 template <int KV, bool QF32>
 cudaError_t launch_kv(const SdpaParams& p, cudaStream_t s) {
   const int group = p.nkv > 0 ? p.n / p.nkv : 0;
-  const bool fast = group >= 1 && group <= 8 && p.n % p.nkv == 0 && p.ws != nullptr &&
+  const bool rows = p.shared_kv && group >= 1 && group <= 8 && p.n % p.nkv == 0 && p.ws != nullptr &&
                     p.ws_bytes >= sdpa_workspace_bytes(p.b, p.n, p.nkv, p.h, p.s_max, p.shared_kv);
-  if (p.q_tiled_out && (!fast || !QF32 || (p.h != 256 && p.h != 128 && p.h != 64)))
+  if (p.q_tiled_out && (!rows || !QF32 || (p.h != 256 && p.h != 128 && p.h != 64)))
     return cudaErrorInvalidValue;  // fused output quantization exists on the fast f32-query path only
-  if (fast && p.h == 256) return launch_fast<KV, 256, QF32>(p, s);
-  if (fast && p.h == 128) return launch_fast<KV, 128, QF32>(p, s);
-  if (fast && p.h == 64) return launch_fast<KV, 64, QF32>(p, s);
+  if (rows && p.h == 256) return launch_rows<KV, 256, QF32>(p, s);
+  if (rows && p.h == 128) return launch_rows<KV, 128, QF32>(p, s);
+  if (rows && p.h == 64) return launch_rows<KV, 64, QF32>(p, s);
   const size_t smem = sizeof(float) * ((size_t)p.h + p.s_max);
   auto kernel = sdpa_decode_generic_kernel<KV, QF32>;
   if (smem > 48 * 1024) {
@@ -1564,15 +1300,21 @@ cudaError_t launch_attn_step_h(const AttnStepParams& p, cudaStream_t s) {
 
 }  // namespace
 
-size_t sdpa_workspace_bytes(int b, int n, int nkv, int h, int s_max, int shared_kv) {
-  (void)n;
+size_t sdpa_chunk_workspace_bytes(int b, int nkv, int h, int s_max, int shared_kv) {
   const int chunk_tokens = pick_chunk_tokens(b, s_max, shared_kv);
   const int chunks_max = (s_max + chunk_tokens - 1) / chunk_tokens;
   // [b][nkv][chunks][8 (query heads of the group, padded)][h + 2] floats
   return (size_t)b * nkv * chunks_max * 8 * partial_stride(h) * sizeof(float);
 }
 
+size_t sdpa_workspace_bytes(int b, int n, int nkv, int h, int s_max, int shared_kv) {
+  (void)n;
+  const size_t chunks = sdpa_chunk_workspace_bytes(b, nkv, h, s_max, shared_kv);
+  return shared_kv ? chunks : std::max(chunks, sdpa_split_workspace_bytes(b, nkv, h, s_max));
+}
+
 cudaError_t launch_sdpa_decode(const SdpaParams& p, cudaStream_t s) {
+  if (sdpa_split_supported(p)) return launch_sdpa_split(p, s);
   const bool qf32 = p.q_dtype == 1;
   switch (p.kv_dtype) {
     case kKvF16: return qf32 ? launch_kv<kKvF16, true>(p, s) : launch_kv<kKvF16, false>(p, s);

@@ -9,7 +9,7 @@
 // caller for a workspace it has no way to obtain; this one brings its own.
 //
 // The split-K partial results live in ONE file-scope device array of
-// kStaticWorkspaceBytes (8 MiB). Every GPU whose context loads this library
+// kStaticArrayBytes (10 MiB). Every GPU whose context loads this library
 // holds that array until the process exits. All calls on a device share it and
 // nothing in it needs clearing between calls (each call writes every record it
 // later reads), but two calls that overlap on the GPU -- different streams, or
@@ -30,10 +30,13 @@
 
 namespace {
 
+// Shapes are admitted by what the chunked record layout takes (b200_sdpa_workspace_bytes), up to this; the split
+// kernels' layout of such a shape is at most 1/33 and 1.3 MB larger, so the array itself is.
 constexpr size_t kStaticWorkspaceBytes = 8u << 20;
+constexpr size_t kStaticArrayBytes = 10u << 20;
 constexpr int kMaxDevices = 64;
 
-static __device__ __align__(256) unsigned char g_sdpa_static_workspace[kStaticWorkspaceBytes];
+static __device__ __align__(256) unsigned char g_sdpa_static_workspace[kStaticArrayBytes];
 
 std::mutex g_mu;
 void* g_device_address[kMaxDevices] = {nullptr};
@@ -90,7 +93,7 @@ int b200_sdpa_decode_static(const void* d_q, const void* d_k, const void* d_v, c
     return static_fail(B200_ERR_INVALID_ARGUMENT, "b200_sdpa_decode_static: int8 cache needs scales");
   // only the split-K kernels use the workspace; other head layouts run on a kernel that needs none
   const bool uses_workspace = n / nkv <= 8 && (h == 64 || h == 128 || h == 256);
-  const size_t need = uses_workspace ? b200::sdpa_workspace_bytes(b, n, nkv, h, s_max) : 0;
+  const size_t need = uses_workspace ? b200::sdpa_chunk_workspace_bytes(b, nkv, h, s_max) : 0;
   if (need > kStaticWorkspaceBytes)
     return static_fail(B200_ERR_UNSUPPORTED,
                        "b200_sdpa_decode_static: this shape needs %zu bytes of workspace, the built-in one holds %zu "
@@ -128,7 +131,7 @@ int b200_sdpa_decode_static(const void* d_q, const void* d_k, const void* d_v, c
   p.scale = scale > 0.0f ? scale : 1.0f / sqrtf((float)h);
   p.logit_cap = logit_cap;
   p.ws = static_cast<float*>(ws);
-  p.ws_bytes = kStaticWorkspaceBytes;
+  p.ws_bytes = kStaticArrayBytes;
   const cudaError_t e = b200::launch_sdpa_decode(p, static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return static_fail(B200_ERR_CUDA, "b200_sdpa_decode_static: %s", cudaGetErrorString(e));
   return B200_OK;

@@ -1,0 +1,107 @@
+"""Kernels that are chosen by size, at the sizes where they can go wrong: edges of tiles and stages, remainders, the
+smallest and the largest of a range. Against plain float64 / integer restatements."""
+import numpy as np
+import pytest
+
+from litert_b200 import workloads
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from litert_b200 import ops as o
+
+    return o
+
+
+@pytest.fixture(scope="module")
+def ws(ops):
+    return ops.Workspace("cuda", 64 << 20)
+
+
+def dev(a):
+    return torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+
+def _attention(q, k, v, length, scale, cap, mask=None):
+    """One row in float64: q [n, h]; k, v [s, nkv, h]."""
+    n, h = q.shape
+    nkv = k.shape[1]
+    out = np.zeros((n, h))
+    if length <= 0:
+        return out
+    for i in range(n):
+        kv = i // (n // nkv)
+        logit = k[:length, kv].astype(np.float64) @ q[i].astype(np.float64) * scale
+        if cap:
+            logit = cap * np.tanh(logit / cap)
+        if mask is not None:
+            logit = logit + mask[:length]
+        p = np.exp(logit - logit.max())
+        out[i] = p @ v[:length, kv].astype(np.float64) / p.sum()
+    return out
+
+
+@pytest.mark.parametrize("kv", ["f16", "i8", "f32"])
+@pytest.mark.parametrize("n,nkv,h", [(8, 1, 256), (6, 2, 128), (4, 4, 64), (3, 1, 64)])
+def test_sdpa_decode_over_unequal_pieces(ops, ws, kv, n, nkv, h):
+    """The cached tokens of all sequences are cut into equal pieces: lengths that end on and next to units (16 tokens),
+    stages (32 to 128) and pieces, empty sequences first, between and last, and rows behind a sequence's last token
+    that hold NaN. Bound: keys, queries, values and weights are fp16 operands (2^-11 each), fp16 outputs another 2^-11:
+    five roundings of 4.9e-4 at most."""
+    rng = np.random.default_rng(n * 100 + h)
+    s_max = 1001
+    lengths = np.asarray([0, 1, 15, 16, 17, 0, 31, 63, 64, 65, 127, 128, 129, 255, 640, 1000, 1001, 0], np.int32)
+    b = len(lengths)
+    q = rng.standard_normal((b, 1, n, h)).astype(np.float32)
+    k = rng.standard_normal((b, s_max, nkv, h)).astype(np.float32)
+    v = rng.standard_normal((b, s_max, nkv, h)).astype(np.float32)
+    kw = dict(scale=1.0 / np.sqrt(h), logit_cap=30.0 if h == 128 else 0.0)
+    mask = None
+    if kv == "i8":
+        kd, ks = workloads.quantize_kv_per_token(k)
+        vd, vs = workloads.quantize_kv_per_token(v)
+        kf, vf = kd.astype(np.float32) * ks[..., None], vd.astype(np.float32) * vs[..., None]
+        kw.update(k_scale=dev(ks), v_scale=dev(vs))
+    else:
+        t = np.float16 if kv == "f16" else np.float32
+        kd, vd = k.astype(t), v.astype(t)
+        kf, vf = kd.astype(np.float32), vd.astype(np.float32)
+        for i, length in enumerate(lengths):
+            kd[i, length:] = np.nan
+            vd[i, length:] = np.nan
+    if kv == "f32":
+        mask = rng.standard_normal((b, s_max)).astype(np.float32)
+        kw["mask"] = dev(mask)
+    else:
+        q = q.astype(np.float16)
+    out = ops.sdpa_decode(dev(q), dev(kd), dev(vd), lengths=dev(lengths), ws=ws, **kw).float().cpu().numpy()
+    ws.check_status()
+    for i, length in enumerate(lengths):
+        want = _attention(q[i, 0].astype(np.float32), kf[i], vf[i], int(length), kw["scale"], kw["logit_cap"],
+                          None if mask is None else mask[i])
+        assert np.max(np.abs(out[i, 0] - want)) <= 5 * 2.0 ** -11 * max(np.max(np.abs(want)), 1e-30), (i, length)
+
+
+@pytest.mark.parametrize("b,s_max,kv", [(1, 5000, "f16"), (1, 63, "i8"), (2, 8192, "i8"), (70, 40, "f16")])
+def test_sdpa_decode_with_many_records_per_sequence_and_many_sequences(ops, ws, b, s_max, kv):
+    """One sequence over all SMs (over 64 records to merge), one piece in all, and more sequences than a warp has lanes."""
+    rng = np.random.default_rng(b + s_max)
+    n, nkv, h = 8, 1, 128
+    q = rng.standard_normal((b, 1, n, h)).astype(np.float16)
+    k = rng.standard_normal((b, s_max, nkv, h)).astype(np.float16)
+    v = rng.standard_normal((b, s_max, nkv, h)).astype(np.float16)
+    lengths = rng.integers(s_max // 2, s_max + 1, b).astype(np.int32)
+    kw = {}
+    kd, vd, kf, vf = k, v, k.astype(np.float32), v.astype(np.float32)
+    if kv == "i8":
+        kd, ks = workloads.quantize_kv_per_token(k)
+        vd, vs = workloads.quantize_kv_per_token(v)
+        kf, vf = kd.astype(np.float32) * ks[..., None], vd.astype(np.float32) * vs[..., None]
+        kw = dict(k_scale=dev(ks), v_scale=dev(vs))
+    out = ops.sdpa_decode(dev(q), dev(kd), dev(vd), lengths=dev(lengths), ws=ws, **kw).float().cpu().numpy()
+    for i in range(b):
+        want = _attention(q[i, 0].astype(np.float32), kf[i], vf[i], int(lengths[i]), 1.0 / np.sqrt(h), 0.0)
+        assert np.max(np.abs(out[i, 0] - want)) <= 5 * 2.0 ** -11 * np.max(np.abs(want)), i
