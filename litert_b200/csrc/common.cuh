@@ -329,6 +329,12 @@ __device__ __forceinline__ void st_async_cluster_u32(uint32_t addr, int32_t v, u
   asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.u32 [%0], %1, [%2];" ::"r"(addr), "r"(v), "r"(remote_bar)
                : "memory");
 }
+__device__ __forceinline__ void st_async_cluster_u32x4(uint32_t addr, int32_t a, int32_t b, int32_t c, int32_t d,
+                                                       uint32_t remote_bar) {  // 16 bytes, addr 16-byte aligned
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(addr), "r"(a),
+               "r"(b), "r"(c), "r"(d), "r"(remote_bar)
+               : "memory");
+}
 __device__ __forceinline__ void st_cluster_u32(uint32_t addr, int32_t v) {
   asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }

@@ -69,11 +69,17 @@ struct UmmaShared {
 #ifndef B200_PER_SM16
 #define B200_PER_SM16 2
 #endif
+#ifndef B200_UMMA_KB32
+#define B200_UMMA_KB32 108
+#endif
+#ifndef B200_PER_SM32
+#define B200_PER_SM32 2
+#endif
 template <int NB>
 struct UmmaBudget {
-  static constexpr int kUmmaKB = NB <= 16 ? B200_UMMA_KB16 : (NB >= 64 ? 206 : 200);
-  static constexpr int kClusterKB = NB <= 16 ? B200_CLUSTER_KB16 : 200;
-  static constexpr int kCtasPerSm = NB <= 16 ? B200_PER_SM16 : 1;
+  static constexpr int kUmmaKB = NB <= 16 ? B200_UMMA_KB16 : (NB == 32 ? B200_UMMA_KB32 : 206);
+  static constexpr int kClusterKB = NB <= 16 ? B200_CLUSTER_KB16 : (NB == 32 ? B200_UMMA_KB32 : 200);
+  static constexpr int kCtasPerSm = NB <= 16 ? B200_PER_SM16 : (NB == 32 ? B200_PER_SM32 : 1);
 };
 
 template <int NB>
@@ -163,11 +169,8 @@ __device__ __forceinline__ void store_output(const FcParams& p, int m, int n, in
 
 
 template <int NB, int EPI>
-__global__ void __launch_bounds__(kUmmaThreads, 1) fc_umma_kernel(const FcParams p, const int m_base_first) {
-  // grid.y = passes of NB activation rows; the stream-K scratch (slots, counters) is numbered over
-  // the whole grid, so every pass merges its own split tiles
-  const int m_base = m_base_first + (int)blockIdx.y * NB;
-  const int cta_base = (int)(blockIdx.y * gridDim.x);
+__global__ void __launch_bounds__(kUmmaThreads, 1) fc_umma_kernel(const FcParams p) {
+  constexpr int m_base = 0;  // one pass of NB activation rows
   using L = UmmaLayout<NB>;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + L::kStages * L::kStageBytes);
@@ -447,6 +450,15 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) fc_umma_kernel(const FcParams
               sc[j] = sh->in_scale[c * 16 + j];
               ax[j] = sh->in_aux[c * 16 + j];
             }
+            if (EPI != kEpiHybridPick && plain) {
+              int32_t* ycol = static_cast<int32_t*>(p.y) + (size_t)(m_base + c * 16) * p.n + n;
+#pragma unroll
+              for (int j = 0; j < 16; ++j) {
+                const int32_t v = compute_output<EPI, true>(p, r[j], rs, wsc, bias_f, base_i, mult, shift, sc[j], ax[j]);
+                if (c * 16 + j < m_valid) ycol[(size_t)j * p.n] = v;
+              }
+              continue;
+            }
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
               const int m = c * 16 + j;
@@ -480,7 +492,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) fc_umma_kernel(const FcParams
         const int c_first = (int)(((tile_first + 1) * g - 1) / total);
         const int c_last = (int)(((tile_last + 1) * g - 1) / total);
         const int which = (t_begin <= tile_first) ? 1 : 0;
-        int32_t* mine = p.ws_part + (size_t)((cta_base + blockIdx.x) * 2 + which) * kZeroWsSlotInts;
+        int32_t* mine = p.ws_part + (size_t)(blockIdx.x * 2 + which) * kZeroWsSlotInts;
 #pragma unroll 1
         for (int c = 0; c < NB / 16; ++c) {
           if (c * 16 >= m_valid) break;
@@ -499,7 +511,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) fc_umma_kernel(const FcParams
         named_barrier(1, kEpiThreads);
         if (etid == 0) {
           __threadfence();
-          const int old = atomicAdd(&p.ws_count[cta_base + c_first], seg_tiles);
+          const int old = atomicAdd(&p.ws_count[c_first], seg_tiles);
           sh->last = (old + seg_tiles == p.k_tiles) ? 1 : 0;
         }
         named_barrier(1, kEpiThreads);
@@ -512,7 +524,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) fc_umma_kernel(const FcParams
             int32_t v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
             for (int c = c_first; c <= c_last; ++c) {
               const int w = (c == c_first) ? 1 : 0;
-              const int32_t* slot = p.ws_part + (size_t)((cta_base + c) * 2 + w) * kZeroWsSlotInts + row_in_tile;
+              const int32_t* slot = p.ws_part + (size_t)(c * 2 + w) * kZeroWsSlotInts + row_in_tile;
 #pragma unroll
               for (int j = 0; j < 8; ++j)
                 if (m0 + j < m_valid) v[j] += __ldcg(slot + (m0 + j) * kTileN);
@@ -525,7 +537,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) fc_umma_kernel(const FcParams
                                     sh->in_aux[m0 + j]);
             }
           }
-          if (etid == 0) p.ws_count[cta_base + c_first] = 0;
+          if (etid == 0) p.ws_count[c_first] = 0;
         }
         named_barrier(1, kEpiThreads);  // sh->last is rewritten by the next split tile
       }
@@ -582,7 +594,8 @@ template <int NB>
 struct ClusterLayout {
   static constexpr int kQBytes = NB * kTileK8;
   static constexpr int kStageBytes = kTileBytes + kQBytes;
-  static constexpr int kRedBytes = (kTileN + 8) * NB * 4;  // split x ceil(128 / split) rows x NB columns of int32
+  static constexpr int kRedPitch = NB + 4;                        // words per row: 16-byte pieces, rows 4 banks apart
+  static constexpr int kRedBytes = (kTileN + 8) * kRedPitch * 4;  // split x ceil(128 / split) rows x NB columns of int32
   static constexpr int kStagesRaw = (UmmaBudget<NB>::kClusterKB * 1024 - kRedBytes) / kStageBytes;
   static constexpr int kStages = kStagesRaw > 10 ? 10 : kStagesRaw;
   static_assert(kStages >= 2, "the ring needs two stages");
@@ -594,10 +607,11 @@ struct ClusterLayout {
 };
 
 template <int NB, int EPI>
-__global__ void __launch_bounds__(kUmmaThreads, 1) fc_cluster_kernel(const FcParams p, const int m_base, const int split) {
+__global__ void __launch_bounds__(kUmmaThreads, 1) fc_cluster_kernel(const FcParams p, const int split) {
   using L = ClusterLayout<NB>;
   extern __shared__ __align__(1024) uint8_t smem[];
-  int32_t* red = reinterpret_cast<int32_t*>(smem + L::kStages * L::kStageBytes);  // [source][column][row in slice]
+  const int m_base = (int)blockIdx.y * NB;  // grid.y = passes of NB activation rows
+  int32_t* red = reinterpret_cast<int32_t*>(smem + L::kStages * L::kStageBytes);  // [source][row in slice][column]
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + L::kStages * L::kStageBytes + L::kRedBytes);
   uint64_t* empty_bar = full_bar + L::kStages;
   uint64_t* acc_full = empty_bar + L::kStages;
@@ -770,14 +784,17 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) fc_cluster_kernel(const FcPar
     // Every int32 sent to an owner also counts as four transaction bytes on the owner's `red_full`
     // barrier (st.async): an owner knows its pieces are in without a second cluster-wide barrier, which
     // cost 0.4 us per launch (measured on B200 against the same exchange with barrier.cluster).
+    // Four columns per message: with one (8192 messages per CTA at 64 rows) the exchange took longer than the
+    // products, 9.8 us of n = k = 2048 at 64 rows against 3.7 at 16.
+    const int cols = m_valid <= 2 ? m_valid : (m_valid + 3) / 4 * 4;
     if (etid == 0) {
       const int owned = min(rows_per_owner, kTileN - rank * rows_per_owner);
-      mbar_arrive_expect_tx(red_full, (uint32_t)(owned > 0 ? split * owned * m_valid * 4 : 0));
+      mbar_arrive_expect_tx(red_full, (uint32_t)(owned > 0 ? split * owned * cols * 4 : 0));
     }
     const uint32_t owner = (uint32_t)(row / rows_per_owner);
     const uint32_t owner_bar = map_to_rank(smem_u32(red_full), owner);
     const uint32_t slot = map_to_rank(smem_u32(red), owner) +
-                          4u * (uint32_t)((rank * NB) * rows_per_owner + row % rows_per_owner);
+                          4u * (uint32_t)((rank * rows_per_owner + row % rows_per_owner) * L::kRedPitch);
 #pragma unroll 1
     for (int c = 0; c < NB / 16; ++c) {
       if (c * 16 >= m_valid) break;
@@ -789,9 +806,15 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) fc_cluster_kernel(const FcPar
 #pragma unroll
         for (int j = 0; j < 16; ++j) r[j] = 0;
       }
+      if (m_valid <= 2) {
 #pragma unroll
-      for (int j = 0; j < 16; ++j)
-        if (c * 16 + j < m_valid) st_async_cluster_u32(slot + 4u * (uint32_t)((c * 16 + j) * rows_per_owner), r[j], owner_bar);
+        for (int j = 0; j < 2; ++j)
+          if (j < m_valid) st_async_cluster_u32(slot + 4u * (uint32_t)j, r[j], owner_bar);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 16; j += 4)
+          if (c * 16 + j < m_valid) st_async_cluster_u32x4(slot + 4u * (uint32_t)(c * 16 + j), r[j], r[j + 1], r[j + 2], r[j + 3], owner_bar);
+      }
     }
     tc_fence_before();
     mbar_wait_bounded(red_full, 0, abort_flag, p.status, kStatusWaitTimeoutTmem);  // everyone's pieces of this CTA's rows
@@ -799,28 +822,38 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) fc_cluster_kernel(const FcPar
     cluster_wait();  // phase 0
   }
   if (warp >= 2 && n_own < p.n) {
-    uint32_t epoch32 = 0;
-    if constexpr (EPI == kEpiHybridF32) {
-      if (p.push_ranks > 1)
-        epoch32 = (uint32_t)(*p.push_step_epoch * (unsigned long long)p.push_per_step + (unsigned long long)p.push_seq + 1ull);
-    }
-    for (int col = col0; col < m_valid; col += col_step) {
+    auto total_of = [&](int col) {
       int32_t v = 0;
-      for (int src = 0; src < split; ++src) v += red[(src * NB + col) * rows_per_owner + r_own];
-      if constexpr (EPI == kEpiHybridF32) {
-        if (p.push_ranks > 1) {
-          // the partial sum goes to every peer as a self-validating message (value and epoch in one 8-byte store)
-          const int32_t bits = compute_output<EPI>(p, v, rs, wsc, bias_f, base_i, mult, shift, sh->in_scale[col], sh->in_aux[col]);
+      for (int src = 0; src < split; ++src) v += red[(src * rows_per_owner + r_own) * L::kRedPitch + col];
+      return v;
+    };
+    bool done = false;
+    if constexpr (EPI == kEpiHybridF32) {
+      if (p.push_ranks > 1) {
+        // the partial sum goes to every peer as a self-validating message (value and epoch in one 8-byte store)
+        const uint32_t epoch32 =
+            (uint32_t)(*p.push_step_epoch * (unsigned long long)p.push_per_step + (unsigned long long)p.push_seq + 1ull);
+        for (int col = col0; col < m_valid; col += col_step) {
+          const int32_t bits =
+              compute_output<EPI>(p, total_of(col), rs, wsc, bias_f, base_i, mult, shift, sh->in_scale[col], sh->in_aux[col]);
           const size_t at = (size_t)(m_base + col) * p.n + n_own;
           static_cast<float*>(p.y)[at] = __int_as_float(bits);
           for (int j = 0; j < p.push_ranks; ++j)
             if (j != p.push_rank)
               asm volatile("st.relaxed.sys.global.v2.u32 [%0], {%1, %2};" ::"l"(p.push_out[j] + at), "r"((uint32_t)bits), "r"(epoch32)
                            : "memory");
-          continue;
         }
+        done = true;
       }
-      store_output<EPI>(p, m_base + col, n_own, v, rs, wsc, bias_f, base_i, mult, shift, sh->in_scale[col], sh->in_aux[col]);
+    }
+    if (!done && plain_epilogue<EPI>(p)) {  // (see compute_output: no branches per output)
+      for (int col = col0; col < m_valid; col += col_step)
+        static_cast<int32_t*>(p.y)[(size_t)(m_base + col) * p.n + n_own] = compute_output<EPI, true>(
+            p, total_of(col), rs, wsc, bias_f, base_i, mult, shift, sh->in_scale[col], sh->in_aux[col]);
+    } else if (!done) {
+      for (int col = col0; col < m_valid; col += col_step)
+        store_output<EPI>(p, m_base + col, n_own, total_of(col), rs, wsc, bias_f, base_i, mult, shift, sh->in_scale[col],
+                          sh->in_aux[col]);
     }
   }
   tc_fence_before();
@@ -848,17 +881,19 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) fc_cluster_kernel(const FcPar
 // slots and runs the epilogue. Integer sums: the result does not depend on the order.
 // Measured on B200, config 2 at M = 512: 86 us one unit per CTA -> 68 persistent -> 63 row parameters
 // preloaded -> 43 with eight epilogue warps -> 35 with the per-output branches hoisted (plain_epilogue).
+template <int NB_>
 struct PrefillLayout {
-  static constexpr int kNB = 256;
+  static constexpr int kNB = NB_;
   static constexpr int kQBytes = kNB * kTileK8;                      // 32 KiB
   static constexpr int kStageBytes = kTileBytes + kQBytes;
-  static constexpr int kStages = 206 * 1024 / kStageBytes;
+  static constexpr int kStagesRaw = (NB_ == 256 ? 206 : 194) * 1024 / kStageBytes;
+  static constexpr int kStages = kStagesRaw > 8 ? 8 : kStagesRaw;
   static constexpr int kEpiWarps = 8;                                 // two per TMEM lane quarter
   static constexpr int kThreads = 64 + 32 * kEpiWarps;
   static constexpr int kOutStageBytes = 2 * 2 * 16 * kTileN * 4;      // two blocks per half of the epilogue warps
   static constexpr int kBarriers = 2 * kStages + 4;
   static constexpr int kSmemBytes = kStages * kStageBytes + kBarriers * 8 + (int)sizeof(UmmaShared) + 32 + kOutStageBytes;
-  static constexpr int kTmemCols = 512;
+  static constexpr int kTmemCols = 2 * NB_;
   static_assert(kSmemBytes <= kMaxDynamicSmem, "prefill kernel: shared memory over the per-CTA limit");
 };
 
@@ -876,10 +911,9 @@ __device__ __forceinline__ PrefillUnit prefill_unit(const FcParams& p, int u, in
   return w;
 }
 
-template <int EPI>
-__global__ void __launch_bounds__(PrefillLayout::kThreads, 1) fc_prefill_kernel(const FcParams p, const int units, const int ksplit) {
-  using L = PrefillLayout;
-  constexpr int NB = L::kNB;
+template <int EPI, int NB>
+__global__ void __launch_bounds__(PrefillLayout<NB>::kThreads, 1) fc_prefill_kernel(const FcParams p, const int units, const int ksplit) {
+  using L = PrefillLayout<NB>;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + L::kStages * L::kStageBytes);
   uint64_t* empty_bar = full_bar + L::kStages;
@@ -1158,11 +1192,11 @@ __global__ void __launch_bounds__(PrefillLayout::kThreads, 1) fc_prefill_kernel(
   if (warp == 1) tmem_dealloc(tmem_base, L::kTmemCols);
 }
 
-template <int EPI>
+template <int EPI, int NB>
 cudaError_t launch_prefill(const FcParams& p, cudaStream_t s) {
-  using L = PrefillLayout;
+  using L = PrefillLayout<NB>;
   static bool configured[64] = {false};
-  auto kernel = fc_prefill_kernel<EPI>;
+  auto kernel = fc_prefill_kernel<EPI, NB>;
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) dev = 0;
@@ -1193,40 +1227,26 @@ cudaError_t launch_prefill(const FcParams& p, cudaStream_t s) {
 // reduction; CTAs with one tile fewer finish early and the kernel stays HBM-bound); with fewer,
 // one SM per n tile cannot pull more than ~80 GB/s, so the flat (n tile, k tile) sequence is cut
 // into equal ranges over all SMs (stream-K) and the partials are merged by the last arriver.
-int plan_ctas(FcParams* p, int passes, int ctas_per_sm) {
+int plan_ctas(FcParams* p, int ctas_per_sm) {
   const int sms = device_sm_count();
   const long long total = (long long)p->n_tiles * p->k_tiles;
   int mode = -1;  // -1 auto, 0 stream-K, 1 whole tiles
   if (const char* e = tuning_env("B200_FC_SPLIT")) mode = atoi(e) ? 0 : 1;  // measurement knob
-  int ctas;
-  if (p->split_passes && passes > 1 && mode != 1) {
-    // few n tiles, a long reduction, several passes of activation rows: the SMs are shared out
-    // among the passes and each pass cuts its (n tile, k tile) sequence into equal ranges
-    p->whole_tiles = 0;
-    ctas = (sms < kZeroWsSlots / 2 ? sms : kZeroWsSlots / 2) / passes;
-  } else if (mode == 1 || passes > 1 || p->force_whole_tiles || (mode < 0 && p->n_tiles * 2 >= sms)) {
-    // (several passes otherwise share one launch as whole n tiles: no cross-CTA reduction)
-    p->whole_tiles = 1;
-    const int cap = passes > 1 ? sms : sms * ctas_per_sm;
-    ctas = p->n_tiles < cap ? p->n_tiles : cap;
-  } else {
-    p->whole_tiles = 0;
-    ctas = sms * ctas_per_sm;
-  }
+  p->whole_tiles = mode == 1 || p->force_whole_tiles || (mode < 0 && p->n_tiles * 2 >= sms);
+  int ctas = sms * ctas_per_sm;
   if (p->max_ctas > 0) ctas = p->max_ctas;
   if (const char* e = tuning_env("B200_FC_MAX_CTAS")) {  // measurement knob
     const int v = atoi(e);
     if (v > 0) ctas = v;
   }
-  if (!p->whole_tiles && ctas * passes > kZeroWsSlots / 2) ctas = kZeroWsSlots / 2 / passes;  // two scratch slots per CTA
+  if (!p->whole_tiles && ctas > kZeroWsSlots / 2) ctas = kZeroWsSlots / 2;  // two scratch slots per CTA
   if (p->whole_tiles && ctas > p->n_tiles) ctas = p->n_tiles;
   if (ctas > total) ctas = (int)total;
-  if (ctas < 1) ctas = 1;
-  return ctas;
+  return ctas < 1 ? 1 : ctas;
 }
 
 template <int NB, int EPI>
-cudaError_t launch_umma_one(const FcParams& p, int m_base, int passes, cudaStream_t s) {
+cudaError_t launch_umma_one(const FcParams& p, cudaStream_t s) {
   using L = UmmaLayout<NB>;
   static bool configured[64] = {false};
   auto kernel = fc_umma_kernel<NB, EPI>;
@@ -1239,24 +1259,13 @@ cudaError_t launch_umma_one(const FcParams& p, int m_base, int passes, cudaStrea
     configured[dev] = true;
   }
   FcParams q = p;
-  const int ctas = plan_ctas(&q, passes, UmmaBudget<NB>::kCtasPerSm);
+  const int ctas = plan_ctas(&q, UmmaBudget<NB>::kCtasPerSm);
   size_t smem = (size_t)L::kSmemBytes;
   if (p.prologue) {
-    if (!fc_prologue_supported(p.m, p.k) || NB != 16 || m_base != 0) return cudaErrorInvalidValue;
+    if (!fc_prologue_supported(p.m, p.k) || NB != 16) return cudaErrorInvalidValue;
     smem += (size_t)p.k_tiles * L::kQBytes;
   }
-  return launch_chained(kernel, dim3(ctas, passes), dim3(kUmmaThreads), smem, s, q, m_base);
-}
-
-template <int EPI>
-cudaError_t launch_umma_nb(const FcParams& p, int m_base, int nb, int passes, cudaStream_t s) {
-  switch (nb) {
-    case 16: return launch_umma_one<16, EPI>(p, m_base, passes, s);
-    case 32: return launch_umma_one<32, EPI>(p, m_base, passes, s);
-    case 64: return launch_umma_one<64, EPI>(p, m_base, passes, s);
-    case 128: return launch_umma_one<128, EPI>(p, m_base, passes, s);
-    default: return launch_umma_one<256, EPI>(p, m_base, passes, s);
-  }
+  return launch_chained(kernel, dim3(ctas), dim3(kUmmaThreads), smem, s, q);
 }
 
 // Largest split of {8, 4, 2} whose clusters all fit on the device at once, 0 when the shape is
@@ -1266,7 +1275,9 @@ int plan_cluster_split(const FcParams& p) {
   if (const char* e = tuning_env("B200_FC_CLUSTER"))  // measurement knob: 0 turns the cluster kernel off
     if (e[0] == '0') return 0;
   const int sms = device_sm_count();
-  if (p.n_tiles * 2 >= sms || p.k_tiles < 2) return 0;
+  const int tiles = p.n_tiles * ((p.m + NB - 1) / NB);
+  constexpr int kPerSm = UmmaBudget<NB>::kCtasPerSm;
+  if (tiles * 2 > sms * kPerSm || p.k_tiles < 2) return 0;
   using L = ClusterLayout<NB>;
   auto kernel = fc_cluster_kernel<NB, EPI>;
   static int capacity[64][17] = {{0}};  // [device][split]: co-resident clusters, -1 = query failed
@@ -1329,7 +1340,7 @@ int plan_cluster_split(const FcParams& p) {
   {
     int big = 12;
     if (const char* e = tuning_env("B200_FC_CLUSTER_BIG")) big = atoi(e);  // measurement knob (0 = off)
-    if (big > 8 && big <= 16 && p.k_tiles >= 8 * big && p.n_tiles * big <= 2 * sms && UmmaBudget<NB>::kCtasPerSm >= 2) {
+    if (big > 8 && big <= 16 && p.k_tiles >= 8 * big && tiles * big <= 2 * sms && kPerSm >= 2) {
       static bool opted[64] = {false};
       if (!opted[dev]) {
         if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
@@ -1341,13 +1352,15 @@ int plan_cluster_split(const FcParams& p) {
       if (opted[dev] && clusters_resident(big) > 0) return big;
     }
   }
-  // the split that puts the most SMs to work with every cluster resident at once
+  // The split that puts the most SMs to work with every cluster resident at once. More tiles than half the SMs (112
+  // tiles of a hidden -> feed-forward layer, say) leave SMs idle as whole tiles and are cut in two or three over two
+  // CTAs per SM: n = 14336, k = 4096 at one row 15.4 us as 112 whole tiles.
   int best = 0;
   for (int split = 8; split >= 2; --split) {
-    if (split > p.k_tiles || p.n_tiles * split > sms) continue;
+    if (split > p.k_tiles || tiles * split > (tiles * 2 > sms ? sms * kPerSm : sms)) continue;
     // (the query counts one CTA per SM; CTAs this small share an SM, and clusters beyond the
     // resident ones simply start as earlier ones finish: nothing waits across clusters)
-    if (clusters_resident(split) * UmmaBudget<NB>::kCtasPerSm >= p.n_tiles) {
+    if (clusters_resident(split) * kPerSm >= tiles) {
       best = split;
       break;
     }
@@ -1356,79 +1369,84 @@ int plan_cluster_split(const FcParams& p) {
 }
 
 template <int NB, int EPI>
-cudaError_t launch_cluster_one(const FcParams& p, int m_base, int split, cudaStream_t s) {
+cudaError_t launch_cluster_one(const FcParams& p, int split, cudaStream_t s) {
   using L = ClusterLayout<NB>;
   size_t smem = (size_t)L::kSmemBytes;
   if (p.prologue) {
-    if (!fc_prologue_supported(p.m, p.k) || NB != 16 || m_base != 0) return cudaErrorInvalidValue;
+    if (!fc_prologue_supported(p.m, p.k) || NB != 16) return cudaErrorInvalidValue;
     smem += (size_t)((p.k_tiles + split - 1) / split + 1) * L::kQBytes;
   }
-  if (p.push_ranks > 1 && (EPI != kEpiHybridF32 || m_base != 0 || !p.push_step_epoch)) return cudaErrorInvalidValue;
-  return launch_chained_cluster(fc_cluster_kernel<NB, EPI>, dim3(p.n_tiles * split), dim3(kUmmaThreads), smem, split, s,
-                                p, m_base, split);
+  if (p.push_ranks > 1 && (EPI != kEpiHybridF32 || p.m > NB || !p.push_step_epoch)) return cudaErrorInvalidValue;
+  return launch_chained_cluster(fc_cluster_kernel<NB, EPI>, dim3(p.n_tiles * split, (p.m + NB - 1) / NB), dim3(kUmmaThreads), smem,
+                                split, s, p, split);
 }
 
-// One pass of nb <= 64 activation rows: the cluster kernel when the shape suits it. Returns
-// cudaErrorNotSupported when the caller should use the stream-K kernel instead.
+// Passes of nb <= 64 activation rows: the cluster kernel when the shape suits it. Returns
+// cudaErrorNotSupported when the caller should use another kernel instead.
 template <int EPI>
-cudaError_t try_cluster_pass(const FcParams& p, int m_base, int nb, cudaStream_t s) {
+cudaError_t try_cluster(const FcParams& p, int nb, cudaStream_t s) {
   int split = 0;
   switch (nb) {
     case 16:
       split = plan_cluster_split<16, EPI>(p);
-      return split ? launch_cluster_one<16, EPI>(p, m_base, split, s) : cudaErrorNotSupported;
+      return split ? launch_cluster_one<16, EPI>(p, split, s) : cudaErrorNotSupported;
     case 32:
       split = plan_cluster_split<32, EPI>(p);
-      return split ? launch_cluster_one<32, EPI>(p, m_base, split, s) : cudaErrorNotSupported;
+      return split ? launch_cluster_one<32, EPI>(p, split, s) : cudaErrorNotSupported;
     case 64:
       split = plan_cluster_split<64, EPI>(p);
-      return split ? launch_cluster_one<64, EPI>(p, m_base, split, s) : cudaErrorNotSupported;
+      return split ? launch_cluster_one<64, EPI>(p, split, s) : cudaErrorNotSupported;
     default:
       return cudaErrorNotSupported;
   }
 }
 
+// Rows per pass of the persistent kernel (64, 128 or 256), by what the launch then costs: waves of (n tile, pass)
+// units, each of which streams k_tiles x (16 KiB of weights + 128 bytes per row) through its SM at the rate L2 gives an
+// SM when all of them pull (80 KB/us; 110 when less than half do) and then stores its outputs. Small passes fill the
+// SMs when there are few n tiles, large ones read the weights fewer times. (Measured at 256 rows per pass whatever the
+// shape: 300 rows of n = 2048, k = 2048 11.8 us, of n = 7360, k = 1536 10.6.)
+int plan_rows_per_pass(const FcParams& p) {
+  const int sms = device_sm_count();
+  int best = 256;
+  double best_us = 1e30;
+  for (int nb = 256; nb >= 64; nb /= 2) {
+    if (p.m_alloc % nb != 0) continue;
+    const int units = p.n_tiles * ((p.m + nb - 1) / nb);
+    int waves = (units + sms - 1) / sms;
+    double kt = p.k_tiles;
+    if (nb == 256 && units * 2 <= sms && p.k_tiles >= 32) {  // launch_prefill cuts the reduction then
+      const int ks = std::min(sms / units, p.k_tiles / 16);
+      if (ks > 1) kt = kt / ks + 16;  // (the merge through memory costs as much as some k tiles)
+    }
+    const double rate = units * 2 < sms ? 110.0 : 80.0;
+    const double us = waves * (kt * (16.0 + nb / 8.0) / rate) + nb * 0.013 + 0.5 * waves;
+    if (us < best_us) best_us = us, best = nb;
+  }
+  return best;
+}
+
 template <int EPI>
 cudaError_t launch_all(const FcParams& p, cudaStream_t s) {
-  int nb = umma_rows_per_pass(p.m);
-  if (nb <= 64) {  // decode-sized: one pass, cluster split-K where the shape suits it
-    const cudaError_t e = try_cluster_pass<EPI>(p, 0, nb, s);
-    if (e != cudaErrorNotSupported) return e;
-    if (p.push_ranks > 1) return cudaErrorInvalidValue;  // only the cluster kernel pushes its outputs to the peers
-    return launch_umma_nb<EPI>(p, 0, nb, 1, s);
+  const int nb = umma_rows_per_pass(p.m);
+  // Decode-sized, and anything else with so few tiles that whole ones would leave half the SMs idle: split-K inside
+  // clusters, up to 64 rows per pass.
+  cudaError_t e = try_cluster<EPI>(p, nb <= 64 ? nb : 64, s);
+  if (e != cudaErrorNotSupported) return e;
+  if (p.push_ranks > 1) return cudaErrorInvalidValue;  // only the cluster kernel pushes its outputs to the peers
+  if (nb == 16) return launch_umma_one<16, EPI>(p, s);
+  if (nb == 32) return launch_umma_one<32, EPI>(p, s);
+  if (nb == 64) return launch_umma_one<64, EPI>(p, s);
+  // Prefill-sized: persistent CTAs over (n tile, pass of activation rows) units.
+  int rows = plan_rows_per_pass(p);
+  if (const char* env = tuning_env("B200_FC_NB")) {  // measurement knob
+    const int v = atoi(env);
+    if (v == 64 || v == 128 || v == 256) rows = v;
   }
-  if (p.push_ranks > 1) return cudaErrorInvalidValue;
-  const int sms = device_sm_count();
-  if (p.m <= 128 && p.n_tiles * 2 < sms && p.m_alloc % 64 == 0) {
-    // a little over one decode pass, few n tiles: 64 rows at a time through the cluster kernel
-    for (int m_base = 0; m_base < p.m; m_base += 64) {
-      const cudaError_t e = try_cluster_pass<EPI>(p, m_base, 64, s);
-      if (e == cudaErrorNotSupported && m_base == 0) break;
-      if (e != cudaSuccess) return e;
-      if (m_base + 64 >= p.m) return cudaSuccess;
-    }
-  }
-  // Prefill-sized: persistent CTAs over (n tile, pass of 256 activation rows) units. (Passes of 128 rows
-  // through the decode kernel, which give twice the CTAs when there are few n tiles, measured no faster
-  // for any shape once the epilogue stopped being the limit: 10.4 against 22.5 us at m = 1024, n = 2560,
-  // k = 2048.) B200_FC_NB=128 keeps that launch for measurements.
-  if (const char* e = tuning_env("B200_FC_NB")) {  // measurement knob
-    const int v = atoi(e);
-    if (v == 128 || v == 256) nb = v;
-  }
-  if (p.m_alloc % nb != 0) return cudaErrorInvalidValue;
-  if (nb == 256) return launch_prefill<EPI>(p, s);
-  const int passes = (p.m + nb - 1) / nb;
-  FcParams q = p;
-  // Whole n tiles per CTA. B200_FC_SPLIT_PASSES=1 (measurement knob) instead shares the SMs out among
-  // the passes and splits each pass's reduction (stream-K): measured slower on B200 for the shapes
-  // that leave SMs idle here (prompt chunk of 512 rows; qkv / o / down projections 26 / 17 / 77 us as
-  // whole tiles, 57 us on average when split): the merge of 128-row partials through memory costs
-  // more than the idle SMs.
-  q.split_passes = 0;
-  if (const char* e = tuning_env("B200_FC_SPLIT_PASSES")) q.split_passes = atoi(e) ? 1 : 0;
-  q.force_whole_tiles = q.split_passes ? 0 : 1;
-  return launch_umma_nb<EPI>(q, 0, nb, passes, s);
+  if (p.m_alloc % rows != 0) return cudaErrorInvalidValue;
+  if (rows == 64) return launch_prefill<EPI, 64>(p, s);
+  if (rows == 128) return launch_prefill<EPI, 128>(p, s);
+  return launch_prefill<EPI, 256>(p, s);
 }
 
 }  // namespace
@@ -1476,7 +1494,7 @@ static cudaError_t launch_pick(const FcParams& p, cudaStream_t s) {
   FcParams q = p;
   q.force_whole_tiles = 1;
   if (fc_argmax_ctas(q.n) > q.argmax_parts) return cudaErrorInvalidValue;
-  return launch_umma_one<16, kEpiHybridPick>(q, 0, 1, s);
+  return launch_umma_one<16, kEpiHybridPick>(q, s);
 }
 
 cudaError_t launch_fc_i8_umma(const FcParams& p, FcEpilogue epi, cudaStream_t s) {

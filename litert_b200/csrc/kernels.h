@@ -97,8 +97,7 @@ struct FcParams {
   int l2_prefetch_tiles;
   int max_ctas;              // 0 = chosen per shape
   int whole_tiles;           // set by the launcher: CTAs own whole n tiles (no split-K)
-  int force_whole_tiles;     // set by the launcher for prefill-sized passes
-  int split_passes;       // several passes in one launch, each split over its share of the SMs (stream-K)
+  int force_whole_tiles;     // set by the launcher: the fused pick wants one slot per CTA
   // Fused greedy pick (hybrid epilogue, at most 16 rows, tcgen05 path): every CTA writes the best value
   // and column of each row among the channels it owns to argmax_val / argmax_idx[row * argmax_parts +
   // CTA] (first index of the maximum, NaN rule of the reference's sampler); soft_cap > 0 replaces a logit
