@@ -356,23 +356,6 @@ struct WarpAttention {
   }
 };
 
-// Ring of shared-memory stages of kRingTokens tokens: every cached row fetched by one bulk asynchronous copy
-// (one row per thread and stage: keys by the lower half of the CTA, values by the upper).
-constexpr int kRingTokens = 64;
-constexpr int kRingStagesMax = 3;
-
-template <int KV, int H>
-struct RingLayout {
-  static constexpr int kRowBytes = H * (KV == kKvI8 ? 1 : 2);
-  static constexpr int kPitch = kRowBytes + 16;  // rows 16 bytes apart in the banks
-  static constexpr int kStageBytes = 2 * kRingTokens * kPitch;
-  static constexpr int kParkBytes = (int)sizeof(float) * kWarps * 8 * (H + 4);
-  static size_t smem_bytes(int stages) {
-    const size_t ring = (size_t)stages * kStageBytes;
-    return (ring > (size_t)kParkBytes ? ring : (size_t)kParkBytes) + 128;
-  }
-};
-
 // Prompt-pass variant (SdpaParams::shared_kv): the rows of the batch are consecutive tokens of ONE
 // sequence and all read the same cache, row b up to lengths[b]. Here a WARP owns a row: the warps of a
 // CTA walk the same chunk of the cache for kWarps neighbouring rows at nearly the same pace, so the
@@ -429,121 +412,342 @@ __global__ void __launch_bounds__(kWarps * 32) sdpa_rows_kernel(const SdpaParams
   }
 }
 
-// Prompt pass with staging (fp16 / int8 caches): a CTA takes kWarps neighbouring rows and one chunk of
-// the shared cache; the chunk goes through the 64-token ring stages of sdpa_decode_ring_kernel ONCE
-// for all the CTA's rows, and every warp runs its own row (its own query, softmax state and partial
-// record) over each stage, masked at the row's own length.
-template <int KV, int H, bool QF32>
-__global__ void __launch_bounds__(kWarps * 32) sdpa_rows_ring_kernel(const SdpaParams p, const int chunk_tokens,
-                                                                     const int chunks_max, const int stages,
-                                                                     const int stage_tokens) {
-  using WA = WarpAttention<KV, H, 4>;  // one pass of 64 tokens per stage
-  using L = RingLayout<KV, H>;
-  constexpr int KSTEPS = WA::KSTEPS;
-  static_assert(WA::kTokensPerWarpIter == kRingTokens, "a warp takes a whole stage per pass");
-  const int stage_bytes = 2 * stage_tokens * L::kPitch;  // (stage_tokens <= kRingTokens: see the decode kernel's launcher)
-  extern __shared__ __align__(128) uint8_t ring_smem[];
-  __shared__ float sm_m[kWarps][8], sm_l[kWarps][8];
-  __shared__ int s_abort;
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(ring_smem);
-  uint8_t* ring = ring_smem + 128;
-  float (*sm_o)[8][H + 4] = reinterpret_cast<float (*)[8][H + 4]>(ring);  // after the loop
-  volatile int* abort_flag = &s_abort;
+// Prompt pass over fp16 / int8 caches. A CTA takes up to 64 (row, query head) pairs of one KV head, neighbouring rows
+// first, and one chunk of the shared cache, 64 tokens at a time: S = Q K^T and O += P V on m16n8k16 with the pairs as
+// the 16-row dimension of a warp (16 pairs each) and tokens, then head dimensions, as the 8-wide one, so that a
+// fragment of K or V serves 16 pairs. K and V have one buffer each: the next keys are fetched under the softmax and
+// P V, the next values under the next Q K^T; 102 KB at H = 256, so that two CTAs share an SM and one's softmax runs under
+// the other's MMAs. int8 rows arrive as bytes and are widened into one fp16 tile that keys and values use in turn.
+// What bounds it is latency: the accumulators leave room for two warps per scheduler, so a step's fragments are requested
+// ahead of the MMAs before, tests that are uniform stay outside the loops over the logits, and every CTA starts with
+// another tile of its chunk (all of them asking L2 for the same lines at once are served in turn).
+// 1024 causal rows, 8 heads x 256, fp16: 65 us with a warp per row and its heads as the 8-wide dimension, 43 us now.
+constexpr int kRowsTile = 64;   // tokens per step
+constexpr int kRowsPairs = 64;  // (row, head) pairs per CTA
 
+template <int KV, int H>
+struct RowsLayout {
+  static constexpr int kPitch = 2 * H + 16;  // fp16 rows 16 bytes apart in the banks: conflict-free ldmatrix
+  static constexpr int kRaw = KV == kKvI8 ? H : 2 * H;
+  static constexpr int kRawPitch = KV == kKvI8 ? H : kPitch;
+  static constexpr int kBarOff = 0;
+  static constexpr int kScaleOff = 32;                                     // [2][64] floats
+  static constexpr int kQOff = kScaleOff + 2 * kRowsTile * 4 + 96;         // (multiples of 128)
+  static constexpr int kKOff = kQOff + kRowsPairs * kPitch;
+  static constexpr int kVOff = kKOff + kRowsTile * kRawPitch;
+  static constexpr int kWideOff = kVOff + kRowsTile * kRawPitch;           // the widened tile of int8 caches
+  static constexpr int kSmemBytes = kWideOff + (KV == kKvI8 ? kRowsTile * kPitch : 0);
+};
+
+__device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr)
+               : "memory");
+}
+__device__ __forceinline__ void ldmatrix4_trans(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr)
+               : "memory");
+}
+// 2^x, weights below the smallest normal number as zero (they become fp16 operands)
+__device__ __forceinline__ float exp2_ftz(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+template <int KV, int H, bool QF32>
+__global__ void __launch_bounds__(kWarps * 32, 2) sdpa_rows_mma_kernel(const SdpaParams p, const int chunk_tokens, const int chunks_max,
+                                                                     const int rows_per_cta) {
+  using L = RowsLayout<KV, H>;
+  extern __shared__ __align__(128) uint8_t rsmem[];
+  __shared__ int s_abort;
+  uint64_t* bar = reinterpret_cast<uint64_t*>(rsmem + L::kBarOff);  // [0] keys, [1] values have arrived
+  float* tok_scale = reinterpret_cast<float*>(rsmem + L::kScaleOff);  // int8: per token of the tile, keys then values
+  volatile int* abort_flag = &s_abort;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int g = lane >> 2, t = lane & 3;
   if (tid == 0) {
-    for (int i = 0; i < kRingStagesMax; ++i) mbar_init(&full_bar[i], 1);
+    mbar_init(&bar[0], 1);
+    mbar_init(&bar[1], 1);
     s_abort = 0;
     mbar_fence_init();
   }
   pdl_enter();
   __syncthreads();
-  const int row0 = (int)blockIdx.z * kWarps, kvh = blockIdx.y, chunk = blockIdx.x;
-  const int b = min(row0 + warp, p.b - 1);          // this warp's row (a surplus warp repeats the last one, unused)
-  const bool row_ok = row0 + warp < p.b;
-  const int b_last = min(row0 + kWarps, p.b) - 1;   // lengths grow with the row: the CTA's longest
-  auto length_of = [&](int r) { return p.lengths ? max(0, min(p.lengths[r], p.s_max)) : p.s_max; };
-  int len_cta = 0;
-  for (int r = row0; r <= b_last; ++r) len_cta = max(len_cta, length_of(r));
-  const int c0 = chunk * chunk_tokens;
-  if (c0 >= len_cta) return;  // uniform over the CTA, nothing in flight
-  const int c1 = min(len_cta, c0 + chunk_tokens);
-  const int len_w = row_ok ? length_of(b) : 0;
-  const int n_sub = (c1 - c0 + stage_tokens - 1) / stage_tokens;
-  const int g = lane >> 2, t = lane & 3;
   const int group = p.n / p.nkv;
-  const typename WA::Rows cache = WA::cache_rows(p, 0, kvh);  // shared_kv: one cache for all rows
+  // the last rows have the longest share of a causal prompt: they start first
+  const int row0 = (int)(gridDim.z - 1 - blockIdx.z) * rows_per_cta, kvh = blockIdx.y, chunk = blockIdx.x;
+  const int n_rows = min(rows_per_cta, p.b - row0);
+  auto length_of = [&](int r) { return p.lengths ? max(0, min(p.lengths[r], p.s_max)) : p.s_max; };
+  int len_max = 0, len_min = p.s_max;
+  for (int r = row0; r < row0 + n_rows; ++r) {
+    const int len = length_of(r);
+    len_max = max(len_max, len);
+    len_min = min(len_min, len);
+  }
+  const int c0 = chunk * chunk_tokens;
+  if (c0 >= len_max) return;  // uniform over the CTA, nothing in flight
+  const int c1 = min(len_max, c0 + chunk_tokens);
+  const int tiles = (c1 - c0 + kRowsTile - 1) / kRowsTile;
 
-  auto issue = [&](int j) {
-    const int s = j % stages;
-    const int t0 = c0 + j * stage_tokens;
-    const int rows = min(stage_tokens, c1 - t0);
-    uint8_t* stage = ring + (size_t)s * stage_bytes;
-    if (tid == 0) mbar_arrive_expect_tx(&full_bar[s], (uint32_t)(2 * rows * L::kRowBytes));
-    const int r = tid & (kRingTokens - 1);
-    if (r < rows) {
-      const bool is_v = tid >= kRingTokens;
-      const uint8_t* src = (is_v ? cache.v : cache.k) + (size_t)(t0 + r) * cache.stride;
-      bulk_g2s(stage + (size_t)(is_v ? stage_tokens : 0) * L::kPitch + (size_t)r * L::kPitch, src, L::kRowBytes, &full_bar[s]);
-    }
+  // one row per thread: keys by the lower half of the CTA, values by the upper. Rows past the end repeat the last
+  // one (their weight is 0).
+  const size_t pitch = (size_t)p.nkv * L::kRaw;
+  const uint8_t* src = static_cast<const uint8_t*>(warp < 2 ? p.k : p.v) + (size_t)kvh * L::kRaw;
+  uint8_t* dst = rsmem + (warp < 2 ? L::kKOff : L::kVOff) + (size_t)(tid & 63) * L::kRawPitch;
+  auto tile_first = [&](int j) { return c0 + (j + (int)blockIdx.z) % tiles * kRowsTile; };
+  auto fetch = [&](int j, int which) {  // (the threads of that half; a phase stays open until its bytes are announced)
+    if (tid == which * 64) mbar_arrive_expect_tx(&bar[which], (uint32_t)(kRowsTile * L::kRaw));
+    bulk_g2s(dst, src + (size_t)min(tile_first(j) + (tid & 63), c1 - 1) * pitch, L::kRaw, &bar[which]);
   };
-  int issued = min(stages, n_sub);
-  for (int j = 0; j < issued; ++j) issue(j);
+  fetch(0, warp >> 1);
 
-  uint32_t qf[KSTEPS][4];
-  {
-    const bool head_ok = g < group;
-    const int head = kvh * group + (head_ok ? g : 0);
-#pragma unroll
-    for (int i = 0; i < KSTEPS; ++i) {
-      const int d0 = 8 * (t + 4 * i);
-      if (!head_ok) {
-        qf[i][0] = qf[i][1] = qf[i][2] = qf[i][3] = 0u;
-      } else if constexpr (QF32) {
-        const float* q = static_cast<const float*>(p.q) + ((size_t)b * p.n + head) * H + d0;
-        load8<kKvF32>(q, 0, true, qf[i]);
+  // ---- Q to shared memory, fp16, pairs as rows ----
+#pragma unroll 8
+  for (int i = tid; i < kRowsPairs * (H / 8); i += kWarps * 32) {
+    const int pair = i / (H / 8), d0 = i % (H / 8) * 8;
+    const int r = pair / group, head = kvh * group + pair % group;
+    uint32_t q[4] = {0u, 0u, 0u, 0u};
+    if (r < n_rows) {
+      if constexpr (QF32) {
+        load8<kKvF32>(static_cast<const float*>(p.q) + ((size_t)(row0 + r) * p.n + head) * H, d0, true, q);
       } else {
-        const __half* q = static_cast<const __half*>(p.q) + ((size_t)b * p.n + head) * H + d0;
-        load8<kKvF16>(q, 0, true, qf[i]);
+        load8<kKvF16>(static_cast<const __half*>(p.q) + ((size_t)(row0 + r) * p.n + head) * H, d0, true, q);
       }
     }
+    *reinterpret_cast<uint4*>(rsmem + L::kQOff + pair * L::kPitch + d0 * 2) = make_uint4(q[0], q[1], q[2], q[3]);
   }
-  WA wa;
-  wa.clear();
-  for (int j = 0; j < n_sub; ++j) {
-    const int s = j % stages;
-    mbar_wait_bounded(&full_bar[s], (uint32_t)(j / stages) & 1u, abort_flag, p.status, kStatusWaitTimeoutFull);
-    const int t0 = c0 + j * stage_tokens;
-    const int t1 = min(min(c1, t0 + stage_tokens), len_w);  // this row's own causal limit
-    if (t0 < t1 && !*abort_flag) {
-      typename WA::Rows rows = cache;
-      const uint8_t* stage = ring + (size_t)s * stage_bytes;
-      rows.k = stage - (ptrdiff_t)t0 * L::kPitch;
-      rows.v = stage + (size_t)stage_tokens * L::kPitch - (ptrdiff_t)t0 * L::kPitch;
-      rows.stride = L::kPitch;
-      wa.template run<kSrcShared>(p, qf, rows, b, t0, kRingTokens, t1, lane, /*fresh=*/false, /*finish=*/false);
-    }
-    __syncthreads();  // every warp is done with stage s
-    if (issued < n_sub && !*abort_flag) {
-      issue(issued);
-      ++issued;
-    }
-  }
-  wa.finish_sums();
-  if (*abort_flag)
-    for (int j = max(0, issued - stages); j < issued; ++j) mbar_drain_bounded(&full_bar[j % stages], (uint32_t)(j / stages) & 1u);
   __syncthreads();
-  wa.park(sm_m, sm_l, sm_o, warp, lane);
-  __syncwarp();
-  if (!row_ok || c0 >= len_w) return;  // (the merge reads only the chunks below the row's length)
-  float* part = p.ws + ((((size_t)b * p.nkv + kvh) * chunks_max + chunk) * 8) * partial_stride(H);
-  for (int idx = lane; idx < group * H; idx += 32) {
-    const int head = idx / H, d = idx % H;
-    float* rec = part + (size_t)head * partial_stride(H);
-    rec[d] = sm_o[warp][head][d];
-    if (d == 0) {
-      rec[H] = sm_m[warp][head];
-      rec[H + 1] = sm_l[warp][head];
+
+  // this thread's pairs: rows g and g + 8 of the warp's 16
+  int len[2], pair_row[2];
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    const int pair = warp * 16 + g + 8 * e;
+    pair_row[e] = pair / group;
+    len[e] = pair_row[e] < n_rows ? length_of(row0 + pair_row[e]) : 0;
+  }
+  const int len_warp = __reduce_max_sync(0xffffffffu, max(len[0], len[1]));
+  const int len_warp_min = __reduce_min_sync(0xffffffffu, min(len[0], len[1]));
+  const float scale_log2 = p.scale * kLog2e;
+  const uint32_t q_addr = smem_u32(rsmem + L::kQOff) + (uint32_t)((warp * 16 + (lane & 15)) * L::kPitch + (lane >> 4) * 16);
+  const uint32_t k_lane = (uint32_t)(((lane & 7) + (lane >> 4) * 8) * L::kPitch + ((lane >> 3) & 1) * 16);
+  const uint32_t v_lane = (uint32_t)((lane & 15) * L::kPitch + (lane >> 4) * 16);
+  const uint32_t k_addr = smem_u32(rsmem + (KV == kKvI8 ? L::kWideOff : L::kKOff)) + k_lane;
+  const uint32_t v_base = smem_u32(rsmem + (KV == kKvI8 ? L::kWideOff : L::kVOff));
+
+  // int8: the raw tile at `off` widened, and the tokens' scales
+  auto widen = [&](int off, const float* scales, float* out, int t0) {
+    for (int i = tid; i < kRowsTile * (H / 8); i += kWarps * 32) {
+      const int r = i / (H / 8), d0 = i % (H / 8) * 8;
+      uint32_t w[4];
+      load8<kKvI8, kSrcGlobalCoherent>(rsmem + off + r * L::kRawPitch, d0, true, w);
+      *reinterpret_cast<uint4*>(rsmem + L::kWideOff + r * L::kPitch + d0 * 2) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+    if (tid < kRowsTile) out[tid] = t0 + tid < c1 ? scales[(size_t)(t0 + tid) * p.nkv + kvh] : 0.0f;
+  };
+
+  float m_run[2] = {-CUDART_INF_F, -CUDART_INF_F}, l_run[2] = {0.0f, 0.0f};
+  float o[H / 8][4];
+#pragma unroll
+  for (int i = 0; i < H / 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.0f;
+
+  for (int j = 0; j < tiles; ++j) {
+    const int t0 = tile_first(j);
+    const bool active = t0 < len_warp;  // uniform over the warp
+    float s[8][4];
+    mbar_wait_bounded(&bar[0], (uint32_t)j & 1u, abort_flag, p.status, kStatusWaitTimeoutFull);
+    if constexpr (KV == kKvI8) {
+      widen(L::kKOff, p.k_scale, tok_scale, t0);
+      __syncthreads();
+      if (warp < 2 && j + 1 < tiles) fetch(j + 1, 0);
+    }
+    if (active) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) s[i][0] = s[i][1] = s[i][2] = s[i][3] = 0.0f;
+      uint32_t a[2][4], b[2][4][4];
+      auto load_step = [&](int kk, int buf) {
+        ldmatrix4(a[buf], q_addr + kk * 32);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) ldmatrix4(b[buf][i], k_addr + i * 16 * L::kPitch + kk * 32);
+      };
+      load_step(0, 0);
+#pragma unroll 4
+      for (int kk = 0; kk < H / 16; ++kk) {
+        const int buf = kk & 1;
+        if (kk + 1 < H / 16) load_step(kk + 1, buf ^ 1);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          mma_f16(s[2 * i], a[buf][0], a[buf][1], a[buf][2], a[buf][3], b[buf][i][0], b[buf][i][1]);
+          mma_f16(s[2 * i + 1], a[buf][0], a[buf][1], a[buf][2], a[buf][3], b[buf][i][2], b[buf][i][3]);
+        }
+      }
+    }
+    if constexpr (KV == kKvF16) {
+      __syncthreads();  // every warp has read the keys
+      if (warp < 2 && j + 1 < tiles) fetch(j + 1, 0);
+    }
+    if (active) {
+      // scale (and dequantise), cap, each row's own limit; online softmax in the log2 domain
+      float mx[2] = {-CUDART_INF_F, -CUDART_INF_F};
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          float f = scale_log2;
+          if constexpr (KV == kKvI8) f *= tok_scale[i * 8 + 2 * t + (e & 1)];
+          s[i][e] *= f;
+        }
+      }
+      if (p.logit_cap > 0.0f) {
+        const float cap = p.logit_cap * kLog2e, ic = 1.0f / cap;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) s[i][e] = cap * tanhf(s[i][e] * ic);
+      }
+      if (t0 + kRowsTile > len_warp_min) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            if (t0 + i * 8 + 2 * t + (e & 1) >= len[e >> 1]) s[i][e] = -CUDART_INF_F;
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) mx[e >> 1] = fmaxf(mx[e >> 1], s[i][e]);
+      float m_use[2], alpha[2];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        float v = mx[e];
+        v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 1));
+        v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 2));
+        const float m_new = fmaxf(m_run[e], v);
+        m_use[e] = m_new == -CUDART_INF_F ? 0.0f : m_new;  // nothing within the limit so far
+        alpha[e] = exp2f(m_run[e] - m_use[e]);
+        m_run[e] = m_new;
+        l_run[e] *= alpha[e];
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          s[i][e] = exp2_ftz(s[i][e] - m_use[e >> 1]);
+          l_run[e >> 1] += s[i][e];
+        }
+      if (__any_sync(0xffffffffu, alpha[0] != 1.0f || alpha[1] != 1.0f)) {  // a maximum has moved
+#pragma unroll
+        for (int i = 0; i < H / 8; ++i) {
+          o[i][0] *= alpha[0];
+          o[i][1] *= alpha[0];
+          o[i][2] *= alpha[1];
+          o[i][3] *= alpha[1];
+        }
+      }
+    }
+    mbar_wait_bounded(&bar[1], (uint32_t)j & 1u, abort_flag, p.status, kStatusWaitTimeoutFull);
+    bool finite = true;
+    if constexpr (KV == kKvI8) {
+      __syncthreads();  // every warp has read the keys' tile
+      widen(L::kVOff, p.v_scale, tok_scale + kRowsTile, t0);
+      __syncthreads();
+      if (warp >= 2 && j + 1 < tiles) fetch(j + 1, 1);
+      if (active) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int c = i * 8 + 2 * t + (e & 1);
+            s[i][e] = t0 + c < len[e >> 1] ? s[i][e] * tok_scale[kRowsTile + c] : 0.0f;
+          }
+      }
+    } else if (t0 + kRowsTile > len_min) {
+      // A tile that some row sees only in part: a value that is not finite would reach that row through 0 x inf, so
+      // such a tile is taken the slow way below.
+      bool ok = true;
+      for (int i = tid; i < kRowsTile * (H / 8); i += kWarps * 32) {
+        const uint4 w = *reinterpret_cast<const uint4*>(rsmem + L::kVOff + (i / (H / 8)) * L::kPitch + i % (H / 8) * 16);
+        const uint32_t ws[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+        for (int q = 0; q < 4; ++q) ok = ok && (ws[q] & 0x7C00u) != 0x7C00u && (ws[q] & 0x7C000000u) != 0x7C000000u;
+      }
+      finite = __syncthreads_and(ok) != 0;
+    }
+    if (active && finite) {
+      uint32_t pa[kRowsTile / 16][4];
+#pragma unroll
+      for (int kk = 0; kk < kRowsTile / 16; ++kk) {
+        pa[kk][0] = pack_half2(s[2 * kk][0], s[2 * kk][1]);
+        pa[kk][1] = pack_half2(s[2 * kk][2], s[2 * kk][3]);
+        pa[kk][2] = pack_half2(s[2 * kk + 1][0], s[2 * kk + 1][1]);
+        pa[kk][3] = pack_half2(s[2 * kk + 1][2], s[2 * kk + 1][3]);
+      }
+      // groups of 64 head dimensions by 16 tokens, the next group's fragments ahead of this one's MMAs
+      constexpr int kGroups = kRowsTile / 16 * (H / 64);
+      uint32_t b[2][4][4];
+      auto load_group = [&](int gi, int buf) {
+        const uint32_t at = v_base + v_lane + (uint32_t)(gi / (H / 64) * 16 * L::kPitch + gi % (H / 64) * 128);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) ldmatrix4_trans(b[buf][i], at + i * 32);
+      };
+      load_group(0, 0);
+#pragma unroll
+      for (int gi = 0; gi < kGroups; ++gi) {
+        const int buf = gi & 1, kk = gi / (H / 64), d = gi % (H / 64) * 8;
+        if (gi + 1 < kGroups) load_group(gi + 1, buf ^ 1);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          mma_f16(o[d + 2 * i], pa[kk][0], pa[kk][1], pa[kk][2], pa[kk][3], b[buf][i][0], b[buf][i][1]);
+          mma_f16(o[d + 2 * i + 1], pa[kk][0], pa[kk][1], pa[kk][2], pa[kk][3], b[buf][i][2], b[buf][i][3]);
+        }
+      }
+    } else if (active) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll 1
+        for (int from = 0; from < 4; ++from)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const int c = i * 8 + 2 * from + e;
+            const float pa = __half2float(__float2half_rn(__shfl_sync(0xffffffffu, s[i][e], (lane & ~3) | from)));
+            const float pb = __half2float(__float2half_rn(__shfl_sync(0xffffffffu, s[i][2 + e], (lane & ~3) | from)));
+            const __half* row = reinterpret_cast<const __half*>(rsmem + L::kVOff + c * L::kPitch);
+            const bool in_a = t0 + c < len[0], in_b = t0 + c < len[1];
+#pragma unroll
+            for (int d = 0; d < H / 8; ++d) {
+              const float2 v = __half22float2(*reinterpret_cast<const __half2*>(row + d * 8 + 2 * t));
+              if (in_a) o[d][0] = fmaf(pa, v.x, o[d][0]), o[d][1] = fmaf(pa, v.y, o[d][1]);
+              if (in_b) o[d][2] = fmaf(pb, v.x, o[d][2]), o[d][3] = fmaf(pb, v.y, o[d][3]);
+            }
+          }
+    }
+    __syncthreads();  // every warp has read the values
+    if constexpr (KV == kKvF16)
+      if (warp >= 2 && j + 1 < tiles) fetch(j + 1, 1);
+  }
+  if (__syncthreads_or(*abort_flag)) {  // never leave with copies in flight
+    mbar_drain_bounded(&bar[0], (uint32_t)(tiles - 1) & 1u);
+    mbar_drain_bounded(&bar[1], (uint32_t)(tiles - 1) & 1u);
+  }
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    l_run[e] += __shfl_xor_sync(0xffffffffu, l_run[e], 1);
+    l_run[e] += __shfl_xor_sync(0xffffffffu, l_run[e], 2);
+  }
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    if (c0 >= len[e]) continue;  // (the merge reads only the chunks below the row's length)
+    const int head = (warp * 16 + g + 8 * e) % group;
+    float* rec = p.ws + (((((size_t)(row0 + pair_row[e]) * p.nkv + kvh) * chunks_max + chunk) * 8) + head) * partial_stride(H);
+#pragma unroll
+    for (int i = 0; i < H / 8; ++i) *reinterpret_cast<float2*>(rec + i * 8 + 2 * t) = make_float2(o[i][2 * e], o[i][2 * e + 1]);
+    if (t == 0) {
+      rec[H] = m_run[e];
+      rec[H + 1] = l_run[e];
     }
   }
 }
@@ -1009,12 +1213,13 @@ __global__ void sdpa_merge_kernel(const SdpaParams p, const int chunk_tokens, co
 // Merge of the per-chunk partials fused with the per-row asymmetric int8 quantization the next
 // hybrid FULLY_CONNECTED applies to the attention output: grid (b), one CTA per sequence over all
 // n*h outputs. Writes the tiled int8 row (+ scale, zero point) and, when p.out is set, the floats.
+// A warp per head, two neighbouring elements per lane and load: 28 -> 14 us for 1024 rows of 8 heads x 256 (a thread per
+// element with up to 16 records each requested ahead was bound by the instructions around its loads).
 template <int H>
 __global__ void __launch_bounds__(1024) sdpa_merge_quant_kernel(const SdpaParams p, const int chunk_tokens,
                                                               const int chunks_max) {
-  extern __shared__ float xs[];        // n * H merged outputs, then n * chunks_max weights
+  extern __shared__ float xs[];        // n * H merged outputs
   __shared__ float red[32];
-  __shared__ float s_linv[64];         // 1 / softmax denominator per head
   pdl_enter();
   const int b = blockIdx.x;
   const int group = p.n / p.nkv;
@@ -1022,71 +1227,43 @@ __global__ void __launch_bounds__(1024) sdpa_merge_quant_kernel(const SdpaParams
   const int chunks = (len + chunk_tokens - 1) / chunk_tokens;
   const size_t cstride = 8 * partial_stride(H);
   const int width = p.n * H;
-  float* wts = xs + width;              // [head][chunk]: exp2(m_chunk - m_head)
-  auto head_base = [&](int head) {
-    const int kvh = head / group, hg = head % group;
-    return p.ws + ((((size_t)b * p.nkv + kvh) * chunks_max) * 8 + hg) * partial_stride(H);
-  };
-  // The partial outputs of this thread's first two elements (first kPre chunks) are requested
-  // before anything else, so that their L2 round trips overlap the per-head statistics below.
-  constexpr int kPre = 16;
-  float pre[2][kPre];
-#pragma unroll
-  for (int e = 0; e < 2; ++e) {
-    const int idx = threadIdx.x + e * blockDim.x;
-    const float* base = idx < width ? head_base(idx / H) + idx % H : nullptr;
-#pragma unroll
-    for (int j = 0; j < kPre; ++j) pre[e][j] = (base && j < chunks) ? base[j * cstride] : 0.0f;
-  }
-  // one warp per head: maximum over the chunks, the chunks' weights and the denominator
+  const int lane = threadIdx.x & 31;
+  float mn = 3.402823466e+38f, mx = -3.402823466e+38f;
   for (int head = threadIdx.x >> 5; head < p.n; head += blockDim.x >> 5) {
-    const int lane = threadIdx.x & 31;
-    const float* base = head_base(head);
+    const int kvh = head / group, hg = head % group;
+    const float* base = p.ws + ((((size_t)b * p.nkv + kvh) * chunks_max) * 8 + hg) * partial_stride(H);
     float mm = -CUDART_INF_F;
     for (int c = lane; c < chunks; c += 32) mm = fmaxf(mm, base[c * cstride + H]);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, o));
     const float muse = mm == -CUDART_INF_F ? 0.0f : mm;
     float l = 0.0f;
-    for (int c = lane; c < chunks; c += 32) {
-      const float f = exp2f(base[c * cstride + H] - muse);
-      wts[head * chunks_max + c] = f;
-      l += f * base[c * cstride + H + 1];
+    float2 acc[H / 64];
+#pragma unroll
+    for (int i = 0; i < H / 64; ++i) acc[i] = make_float2(0.0f, 0.0f);
+#pragma unroll 4
+    for (int c = 0; c < chunks; ++c) {
+      const float* rec = base + c * cstride;
+      const float2 ml = *reinterpret_cast<const float2*>(rec + H);
+      const float w = exp2f(ml.x - muse);
+      l += w * ml.y;
+#pragma unroll
+      for (int i = 0; i < H / 64; ++i) {
+        const float2 v = *reinterpret_cast<const float2*>(rec + i * 64 + 2 * lane);
+        acc[i].x += w * v.x;
+        acc[i].y += w * v.y;
+      }
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-    if (lane == 0) s_linv[head & 63] = l;
-  }
-  __syncthreads();
-  float mn = 3.402823466e+38f, mx = -3.402823466e+38f;
-  int e = 0;
-  for (int idx = threadIdx.x; idx < width; idx += blockDim.x, ++e) {
-    const int head = idx / H, d = idx % H;
-    const float* base = head_base(head) + d;
-    const float* w = wts + head * chunks_max;
-    float acc = 0.0f;
-    int c = 0;
-    if (e < 2) {
-      const int npre = chunks < kPre ? chunks : kPre;
-#pragma unroll
-      for (int j = 0; j < kPre; ++j)
-        if (j < npre) acc += w[j] * (e == 0 ? pre[0][j] : pre[1][j]);
-      c = npre;
+    for (int i = 0; i < H / 64; ++i) {
+      // an empty sequence gives a zero row
+      const float2 v = l > 0.0f ? make_float2(acc[i].x / l, acc[i].y / l) : make_float2(0.0f, 0.0f);
+      const int idx = head * H + i * 64 + 2 * lane;
+      *reinterpret_cast<float2*>(xs + idx) = v;
+      if (p.out) *reinterpret_cast<float2*>(static_cast<float*>(p.out) + (size_t)b * width + idx) = v;
+      mn = fminf(mn, fminf(v.x, v.y));
+      mx = fmaxf(mx, fmaxf(v.x, v.y));
     }
-    for (; c + 8 <= chunks; c += 8) {   // eight independent loads in flight per thread
-      float a[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) a[j] = base[(c + j) * cstride];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) acc += w[c + j] * a[j];
-    }
-    for (; c < chunks; ++c) acc += w[c] * base[c * cstride];
-    const float l = s_linv[head & 63];
-    const float v = l > 0.0f ? acc / l : 0.0f;  // an empty sequence gives a zero row
-    xs[idx] = v;
-    if (p.out) static_cast<float*>(p.out)[(size_t)b * width + idx] = v;
-    mn = fminf(mn, v);
-    mx = fmaxf(mx, v);
   }
   const int k_pad = (width + 127) / 128 * 128;
   quantize_smem_row(xs, width, k_pad, b, p.m_alloc, mn, mx, p.q_tiled_out, p.out_scales, p.out_zps, red);
@@ -1177,44 +1354,35 @@ int pick_chunk_tokens(int b, int s_max, int shared_kv) {
 
 template <int KV, int H, bool QF32>
 cudaError_t launch_rows(const SdpaParams& p, cudaStream_t s) {
-  const int chunk_tokens = pick_chunk_tokens(p.b, p.s_max, p.shared_kv);
-  const int chunks_max = (p.s_max + chunk_tokens - 1) / chunk_tokens;
+  int chunk_tokens = pick_chunk_tokens(p.b, p.s_max, p.shared_kv);
+  int chunks_max = (p.s_max + chunk_tokens - 1) / chunk_tokens;
   cudaError_t e;
   bool staged = false;
-  static const bool ring_env = [] {  // B200_SDPA_RING=0: measurement knob, keeps the register-fed kernel
-    const char* e = tuning_env("B200_SDPA_RING");
-    return !(e && e[0] == '0');
-  }();
   if constexpr (KV != kKvF32) {
-    const bool aligned = ((reinterpret_cast<uintptr_t>(p.k) | reinterpret_cast<uintptr_t>(p.v)) & 15) == 0;
-    if (ring_env && aligned && chunk_tokens % kRingTokens == 0) {
-      using L = RingLayout<KV, H>;
-      // Whole 64-token stages here, even when only one fits: a warp's pass covers 64 tokens, and this kernel
-      // is bound by its arithmetic, not by the copies (1024-token prompt, fp16 rows, measured per layer:
-      // 65.7 us with one 64-token stage, 75.8 with two of 48, 90.2 with three of 32).
-      int stage_tokens = kRingTokens;
-      static const int rtokens_env = [] {  // B200_ROWS_STAGE_TOKENS: measurement knob
-        const char* e = tuning_env("B200_ROWS_STAGE_TOKENS");
-        return e ? atoi(e) : 0;
-      }();
-      if (rtokens_env == 16 || rtokens_env == 32 || rtokens_env == 48 || rtokens_env == 64) stage_tokens = rtokens_env;
-      const int stage_bytes = 2 * stage_tokens * L::kPitch;
-      int stages = std::min(kRingStagesMax, (chunk_tokens + stage_tokens - 1) / stage_tokens);
-      stages = std::min(stages, std::max(1, (104 * 1024) / stage_bytes));
-      const size_t ring_bytes = (size_t)stages * stage_bytes;
-      const size_t smem = (ring_bytes > (size_t)L::kParkBytes ? ring_bytes : (size_t)L::kParkBytes) + 128;
-      auto kernel = sdpa_rows_ring_kernel<KV, H, QF32>;
+    const bool aligned = ((reinterpret_cast<uintptr_t>(p.k) | reinterpret_cast<uintptr_t>(p.v) | reinterpret_cast<uintptr_t>(p.q) |
+                           reinterpret_cast<uintptr_t>(p.ws)) & 15) == 0;
+    if (aligned && !p.mask) {
+      using L = RowsLayout<KV, H>;
+      const int rows_per_cta = kRowsPairs / (p.n / p.nkv);
+      const int groups = (p.b + rows_per_cta - 1) / rows_per_cta * p.nkv;
+      // A step of 64 tokens takes a CTA its latency whatever else the SM does, so the chunks are short enough for two CTAs
+      // on each SM (causal prompts: a third of them have nothing to do) and no shorter, since every chunk leaves a record
+      // per row. Never below pick_chunk_tokens', which sizes the workspace. 1024 rows, 8 heads x 256, with the merge:
+      // chunks of 256 / 320 / 384 tokens 64 / 59 / 64 us.
+      if (groups * ((p.s_max + 319) / 320) >= 2 * device_sm_count()) chunk_tokens = 320;
+      chunks_max = (p.s_max + chunk_tokens - 1) / chunk_tokens;
+      auto kernel = sdpa_rows_mma_kernel<KV, H, QF32>;
       static bool configured[64] = {false};
       int dev = 0;
       cudaGetDevice(&dev);
       if (dev < 0 || dev >= 64) dev = 0;
       if (!configured[dev]) {
-        cudaError_t ea = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::smem_bytes(kRingStagesMax));
+        cudaError_t ea = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kSmemBytes);
         if (ea != cudaSuccess) return ea;
         configured[dev] = true;
       }
-      const dim3 rgrid(chunks_max, p.nkv, (p.b + kWarps - 1) / kWarps);
-      e = launch_chained(kernel, rgrid, dim3(kWarps * 32), smem, s, p, chunk_tokens, chunks_max, stages, stage_tokens);
+      e = launch_chained(kernel, dim3(chunks_max, p.nkv, (p.b + rows_per_cta - 1) / rows_per_cta), dim3(kWarps * 32), (size_t)L::kSmemBytes,
+                         s, p, chunk_tokens, chunks_max, rows_per_cta);
       staged = true;
     }
   }
@@ -1238,7 +1406,7 @@ cudaError_t launch_rows(const SdpaParams& p, cudaStream_t s) {
   if (e != cudaSuccess) return e;
   if (p.q_tiled_out) {
     if (p.n > 64) return cudaErrorInvalidValue;
-    const size_t smem = sizeof(float) * ((size_t)p.n * H + (size_t)p.n * chunks_max);
+    const size_t smem = sizeof(float) * (size_t)p.n * H;
     if (smem > 48 * 1024) {
       cudaError_t ea = cudaFuncSetAttribute(sdpa_merge_quant_kernel<H>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (ea != cudaSuccess) return ea;

@@ -105,3 +105,37 @@ def test_sdpa_decode_with_many_records_per_sequence_and_many_sequences(ops, ws, 
     for i in range(b):
         want = _attention(q[i, 0].astype(np.float32), kf[i], vf[i], int(lengths[i]), 1.0 / np.sqrt(h), 0.0)
         assert np.max(np.abs(out[i, 0] - want)) <= 5 * 2.0 ** -11 * np.max(np.abs(want)), i
+
+
+@pytest.mark.parametrize("kv", ["f16", "i8"])
+@pytest.mark.parametrize("n,nkv,h,s_max", [(8, 1, 256, 1100), (7, 1, 128, 700), (6, 2, 64, 130), (4, 4, 256, 64)])
+def test_sdpa_rows_of_any_lengths(ops, kv, n, nkv, h, s_max):
+    """Query tokens that share one cache, in no order of their lengths: limits on and next to tiles (64 tokens) and
+    chunks (256, 320), empty rows, a last CTA that is not full, and cached values that are not finite behind some rows'
+    limits. Bound as for the decode step: five roundings of 2^-11."""
+    rng = np.random.default_rng(n * 100 + h)
+    marks = [0, 1, 63, 64, 65, 127, 128, 129, 255, 256, 257, 319, 320, 321, 640, 1024, s_max - 1, s_max]
+    lengths = np.asarray([m for m in marks if m <= s_max] + list(rng.integers(1, s_max + 1, 83)), np.int32)
+    rng.shuffle(lengths)
+    rows = len(lengths)
+    q = rng.standard_normal((rows, n, h)).astype(np.float16)
+    k = rng.standard_normal((s_max, nkv, h)).astype(np.float16)
+    v = rng.standard_normal((s_max, nkv, h)).astype(np.float16)
+    kw = dict(scale=1.0 / np.sqrt(h), logit_cap=30.0 if h == 128 else 0.0)
+    bad = s_max
+    if kv == "i8":
+        kd, ks = (a[0] for a in workloads.quantize_kv_per_token(k[None]))
+        vd, vs = (a[0] for a in workloads.quantize_kv_per_token(v[None]))
+        kf, vf = kd.astype(np.float32) * ks[..., None], vd.astype(np.float32) * vs[..., None]
+        kw.update(k_scale=dev(ks), v_scale=dev(vs))
+    else:
+        bad = s_max * 3 // 4 + 5  # a token whose value is not finite
+        v[bad, :, ::3] = np.inf
+        kd, vd, kf, vf = k, v, k.astype(np.float32), v.astype(np.float32)
+    out = ops.sdpa_rows(dev(q), dev(kd), dev(vd), dev(lengths), **kw).float().cpu().numpy()
+    for i, length in enumerate(lengths):
+        if length > bad:
+            assert not np.isfinite(out[i, :, ::3]).any() and np.isfinite(out[i, :, 1::3]).all()
+            continue
+        want = _attention(q[i].astype(np.float32), kf, vf, int(length), kw["scale"], kw["logit_cap"])
+        assert np.max(np.abs(out[i] - want)) <= 5 * 2.0 ** -11 * max(np.max(np.abs(want)), 1e-30), (i, length)
