@@ -329,6 +329,93 @@ __device__ __forceinline__ float gelu_tanh(float v) {
   return __fmul_rn(__fmul_rn(0.5f, v), __fadd_rn(1.0f, th));
 }
 
+// The same over many rows (a prompt chunk): a row's elements stay in the registers of 256 threads, all requested at once,
+// four neighbours per thread and load; one trip to memory and three barriers per row instead of four dependent trips
+// through shared memory. With the rotation below, a prompt of 1024 tokens 5993 -> 5745 us (12.5 us a norm before). Rows of up to 1024 VECS elements that start on 16-byte boundaries.
+template <int VECS>
+__global__ void __launch_bounds__(256) add_norm_quant_rows_kernel(float* __restrict__ h, const float* __restrict__ delta,
+                                                                  const float* __restrict__ gain, int d, int d_pad, float eps,
+                                                                  int m_alloc, int8_t* __restrict__ q_tiled,
+                                                                  float* __restrict__ scales, int32_t* __restrict__ zps) {
+  __shared__ float red[32];
+  __shared__ float2 s_mm[32];
+  __shared__ float s_inv;
+  __shared__ int s_zp, s_zero;
+  pdl_launch_dependents();
+  const int b = blockIdx.x;
+  float* hr = h + (size_t)b * d;
+  float4 gv[VECS], v[VECS];
+#pragma unroll
+  for (int j = 0; j < VECS; ++j) {
+    const int i = (j * 256 + (int)threadIdx.x) * 4;
+    gv[j] = i < d ? *reinterpret_cast<const float4*>(gain + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  }
+  pdl_wait();
+#pragma unroll
+  for (int j = 0; j < VECS; ++j) {
+    const int i = (j * 256 + (int)threadIdx.x) * 4;
+    v[j] = i < d ? __ldcg(reinterpret_cast<const float4*>(hr + i)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  }
+  if (delta) {
+    float4 e[VECS];
+#pragma unroll
+    for (int j = 0; j < VECS; ++j) {
+      const int i = (j * 256 + (int)threadIdx.x) * 4;
+      if (i < d) e[j] = __ldcg(reinterpret_cast<const float4*>(delta + (size_t)b * d + i));
+    }
+#pragma unroll
+    for (int j = 0; j < VECS; ++j) {
+      const int i = (j * 256 + (int)threadIdx.x) * 4;
+      if (i >= d) continue;
+      v[j] = make_float4(__fadd_rn(v[j].x, e[j].x), __fadd_rn(v[j].y, e[j].y), __fadd_rn(v[j].z, e[j].z), __fadd_rn(v[j].w, e[j].w));
+      *reinterpret_cast<float4*>(hr + i) = v[j];
+    }
+  }
+  float ss = 0.0f;
+#pragma unroll
+  for (int j = 0; j < VECS; ++j) {
+    ss += v[j].x * v[j].x;
+    ss += v[j].y * v[j].y;
+    ss += v[j].z * v[j].z;
+    ss += v[j].w * v[j].w;
+  }
+  ss = block_reduce(ss, [](float a, float c) { return a + c; }, 0.0f, red);
+  const float inv_rms = 1.0f / sqrtf(ss / (float)d + eps);
+  float mn = 3.402823466e+38f, mx = -3.402823466e+38f;
+#pragma unroll
+  for (int j = 0; j < VECS; ++j) {
+    if ((j * 256 + (int)threadIdx.x) * 4 >= d) continue;
+    v[j].x = __fmul_rn(__fmul_rn(v[j].x, inv_rms), gv[j].x);
+    v[j].y = __fmul_rn(__fmul_rn(v[j].y, inv_rms), gv[j].y);
+    v[j].z = __fmul_rn(__fmul_rn(v[j].z, inv_rms), gv[j].z);
+    v[j].w = __fmul_rn(__fmul_rn(v[j].w, inv_rms), gv[j].w);
+    mn = fminf(fminf(mn, fminf(v[j].x, v[j].y)), fminf(v[j].z, v[j].w));
+    mx = fmaxf(fmaxf(mx, fmaxf(v[j].x, v[j].y)), fmaxf(v[j].z, v[j].w));
+  }
+  block_minmax(mn, mx, s_mm);
+  if (threadIdx.x == 0) {
+    float sf, inv;
+    int zp, zero_row;
+    row_quant_params(mn, mx, true, &sf, &inv, &zp, &zero_row);
+    s_inv = inv, s_zp = zp, s_zero = zero_row;
+    scales[b] = sf;
+    zps[b] = zp;
+  }
+  __syncthreads();
+  const bool zero = s_zero != 0;
+  const float inv = s_inv, zpf = (float)s_zp;
+#pragma unroll
+  for (int j = 0; j < VECS; ++j) {
+    const int i = (j * 256 + (int)threadIdx.x) * 4;
+    if (i >= d_pad) continue;
+    uint32_t word = 0;
+    if (i < d && !zero)
+      word = quantize_value(v[j].x, inv, zpf, true) | quantize_value(v[j].y, inv, zpf, true) << 8 |
+             quantize_value(v[j].z, inv, zpf, true) << 16 | quantize_value(v[j].w, inv, zpf, true) << 24;
+    *reinterpret_cast<uint32_t*>(q_tiled + q_tiled_offset(b, i, m_alloc)) = word;
+  }
+}
+
 // f = gelu_tanh(gate) * up from the fused projection output [b, 2 f]; quantize f per row.
 // A row (16384 elements at the benchmark's size) is spread over a cluster of kGegluCluster CTAs:
 // each computes its slice into shared memory with its local min / max, the CTAs exchange those
@@ -480,6 +567,81 @@ __global__ void rope_cache_kernel(const float* __restrict__ qkv, int heads, int 
   }
 }
 
+// The same over many rows (a prompt chunk): a warp per (row, head), four neighbouring rotation pairs per lane, so that a
+// row of 256 is two loads of 16 bytes per lane and there is no block to launch or to synchronise per head. Head sizes of
+// 128 or 256 (half / 4 lanes at work), all pointers on 16-byte boundaries.
+template <bool KV_I8>
+__global__ void __launch_bounds__(256) rope_cache_rows_kernel(const float* __restrict__ qkv, int batch, int heads, int kv_heads,
+                                                              int head_dim, const float2* __restrict__ rope_cs,
+                                                              const int32_t* __restrict__ positions, int max_seq,
+                                                              float* __restrict__ q_out, void* __restrict__ k_cache,
+                                                              void* __restrict__ v_cache, float* __restrict__ k_scale,
+                                                              float* __restrict__ v_scale, int one_sequence) {
+  pdl_enter();
+  const int slots = heads + 2 * kv_heads;
+  const int unit = (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5));
+  if (unit >= batch * slots) return;
+  const int b = unit / slots, slot = unit % slots, half = head_dim / 2, i = (int)(threadIdx.x & 31) * 4;
+  const bool in = i < half;
+  const float* src = qkv + (size_t)unit * head_dim;
+  float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f), c = a;
+  if (in) a = *reinterpret_cast<const float4*>(src + i), c = *reinterpret_cast<const float4*>(src + half + i);
+  const int pos = positions[b];
+  float x1[4] = {a.x, a.y, a.z, a.w}, x2[4] = {c.x, c.y, c.z, c.w};
+  const bool is_v = slot >= heads + kv_heads;
+  if (!is_v && in) {
+    const float4* cs = reinterpret_cast<const float4*>(rope_cs + (size_t)min(pos, max_seq) * half + i);
+    const float4 r0 = cs[0], r1 = cs[1];
+    const float co[4] = {r0.x, r0.z, r1.x, r1.z}, si[4] = {r0.y, r0.w, r1.y, r1.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float lo = __fsub_rn(__fmul_rn(x1[e], co[e]), __fmul_rn(x2[e], si[e]));
+      const float hi = __fadd_rn(__fmul_rn(x2[e], co[e]), __fmul_rn(x1[e], si[e]));
+      x1[e] = lo;
+      x2[e] = hi;
+    }
+  }
+  if (slot < heads) {
+    float* dst = q_out + ((size_t)b * heads + slot) * head_dim;
+    if (in) {
+      *reinterpret_cast<float4*>(dst + i) = make_float4(x1[0], x1[1], x1[2], x1[3]);
+      *reinterpret_cast<float4*>(dst + half + i) = make_float4(x2[0], x2[1], x2[2], x2[3]);
+    }
+    return;
+  }
+  const int kvh = is_v ? slot - heads - kv_heads : slot - heads;
+  if (pos >= max_seq) return;  // cache full: the step is ignored for this sequence
+  const size_t tok = ((size_t)(one_sequence ? 0 : b) * max_seq + pos) * kv_heads + kvh;
+  if constexpr (KV_I8) {
+    // symmetric per token and kv head: scale = max|row| / 127
+    float amax = 0.0f;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) amax = fmaxf(amax, fmaxf(fabsf(x1[e]), fabsf(x2[e])));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    const float sc = amax > 0.0f ? __fdiv_rn(amax, 127.0f) : 1.0f;
+    int8_t* dst = static_cast<int8_t*>(is_v ? v_cache : k_cache) + tok * head_dim;
+    uint32_t lo = 0, hi = 0;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      lo |= (uint32_t)(uint8_t)(int8_t)max(-127, min(127, __float2int_rn(__fdiv_rn(x1[e], sc)))) << (8 * e);
+      hi |= (uint32_t)(uint8_t)(int8_t)max(-127, min(127, __float2int_rn(__fdiv_rn(x2[e], sc)))) << (8 * e);
+    }
+    if (in) {
+      *reinterpret_cast<uint32_t*>(dst + i) = lo;
+      *reinterpret_cast<uint32_t*>(dst + half + i) = hi;
+    }
+    if (i == 0) (is_v ? v_scale : k_scale)[tok] = sc;
+  } else if (in) {
+    __half* dst = static_cast<__half*>(is_v ? v_cache : k_cache) + tok * head_dim;
+    __half2 w[4];
+    w[0] = __floats2half2_rn(x1[0], x1[1]), w[1] = __floats2half2_rn(x1[2], x1[3]);
+    w[2] = __floats2half2_rn(x2[0], x2[1]), w[3] = __floats2half2_rn(x2[2], x2[3]);
+    *reinterpret_cast<uint2*>(dst + i) = *reinterpret_cast<const uint2*>(&w[0]);
+    *reinterpret_cast<uint2*>(dst + half + i) = *reinterpret_cast<const uint2*>(&w[2]);
+  }
+}
+
 // grid (parts, b): each CTA scans a slice of the row.
 __global__ void __launch_bounds__(256) argmax_partial_kernel(const float* __restrict__ logits, int n, int parts,
                                                              float soft_cap, float* __restrict__ part_val,
@@ -591,6 +753,12 @@ cudaError_t launch_add_norm_quant(float* h, const float* delta, const float* gai
       (reinterpret_cast<uintptr_t>(delta) & 7) == 0 && (reinterpret_cast<uintptr_t>(gain) & 7) == 0 && !tuning_env("B200_NORM_STAGED"))
     return launch_chained(add_norm_quant_pair_kernel, dim3(batch), dim3(kNormThreads), 0, s, h, delta, gain, d, d_pad, eps, m_alloc,
                           q_tiled, scales, zps, x);
+  const bool vec = d % 4 == 0 && ((reinterpret_cast<uintptr_t>(h) | reinterpret_cast<uintptr_t>(delta) |
+                                   reinterpret_cast<uintptr_t>(gain)) & 15) == 0;
+  if (many && vec && x.tp_size <= 1 && d_pad <= 4096) {
+    auto kernel = d_pad <= 1024 ? add_norm_quant_rows_kernel<1> : d_pad <= 2048 ? add_norm_quant_rows_kernel<2> : add_norm_quant_rows_kernel<4>;
+    return launch_chained(kernel, dim3(batch), dim3(256), 0, s, h, delta, gain, d, d_pad, eps, m_alloc, q_tiled, scales, zps);
+  }
   int batched = 1;
   if (const char* e = tuning_env("B200_NORM_BATCHED")) batched = atoi(e);  // measurement knob
   return launch_chained(add_norm_quant_kernel, dim3(batch), dim3(many ? 256 : kNormThreads), sizeof(float) * d, s, h, delta, gain,
@@ -632,6 +800,14 @@ cudaError_t launch_geglu_quant(const float* gate_up, int batch, int f, int m_all
 cudaError_t launch_rope_cache(const float* qkv, int batch, int heads, int kv_heads, int head_dim, const float2* rope_cs,
                               const int32_t* positions, int max_seq, float* q_out, void* k_cache, void* v_cache,
                               float* k_scale, float* v_scale, int kv_int8, int one_sequence, cudaStream_t s) {
+  const bool aligned = ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(rope_cs) | reinterpret_cast<uintptr_t>(q_out) |
+                         reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache)) & 15) == 0;
+  if (batch > kLatencyRows && aligned && (head_dim == 128 || head_dim == 256)) {
+    const dim3 blocks((unsigned)(((long long)batch * (heads + 2 * kv_heads) + 7) / 8));
+    auto kernel = kv_int8 ? rope_cache_rows_kernel<true> : rope_cache_rows_kernel<false>;
+    return launch_chained(kernel, blocks, dim3(256), 0, s, qkv, batch, heads, kv_heads, head_dim, rope_cs, positions, max_seq, q_out,
+                          k_cache, v_cache, k_scale, v_scale, one_sequence);
+  }
   dim3 grid(batch, heads + 2 * kv_heads);
   if (kv_int8) {
     return launch_chained(rope_cache_kernel<true>, grid, dim3(head_dim / 2), 0, s, qkv, heads, kv_heads, head_dim, rope_cs,

@@ -139,3 +139,44 @@ def test_sdpa_rows_of_any_lengths(ops, kv, n, nkv, h, s_max):
             continue
         want = _attention(q[i].astype(np.float32), kf, vf, int(length), kw["scale"], kw["logit_cap"])
         assert np.max(np.abs(out[i] - want)) <= 5 * 2.0 ** -11 * max(np.max(np.abs(want)), 1e-30), (i, length)
+
+
+@pytest.mark.parametrize("d", [4, 1000, 1024, 1028, 2048, 2052, 4096])
+def test_norm_of_many_rows_equals_that_of_a_few(ops, d):
+    """33 rows and more are kept in registers, four neighbours per thread: widths on and next to a thread's pieces.
+    Residuals are equal; the sum of squares is added in another order (relative error up to d 2^-24), so a scale may
+    differ by that and an integer by one where a value lies on a rounding boundary."""
+    rng = np.random.default_rng(d)
+    h = rng.standard_normal((40, d)).astype(np.float32) * 3
+    delta, gain = rng.standard_normal((40, d)).astype(np.float32), rng.uniform(0.9, 1.1, d).astype(np.float32)
+    many = dev(h)
+    got = ops.add_rmsnorm_quantize(many, dev(delta), dev(gain))
+    for r in range(0, 40, 20):
+        few = dev(h[r:r + 20])
+        want = ops.add_rmsnorm_quantize(few, dev(delta[r:r + 20]), dev(gain))
+        assert torch.equal(few, many[r:r + 20])
+        assert torch.allclose(got.scales[r:r + 20], want.scales[:20], rtol=d * 2.0 ** -24, atol=0)
+        assert torch.equal(got.zero_points[r:r + 20], want.zero_points[:20])
+        diff = (got.rows()[r:r + 20].int() - want.rows()[:20].int()).abs()
+        assert int(diff.max()) <= 1 and float((diff != 0).float().mean()) <= 1e-3
+
+
+@pytest.mark.parametrize("kv", ["f16", "i8"])
+@pytest.mark.parametrize("heads,kv_heads,h", [(8, 1, 256), (6, 2, 128), (3, 3, 128)])
+def test_rotation_of_many_rows_equals_that_of_a_few(ops, kv, heads, kv_heads, h):
+    """33 rows and more take a warp per (row, head): the same bits as a block per (row, head)."""
+    rng = np.random.default_rng(heads)
+    rows, max_seq = 45, 50
+    qkv = rng.standard_normal((rows, (heads + 2 * kv_heads) * h)).astype(np.float32)
+    pos = (np.arange(rows) + 8).astype(np.int32)  # the last three lie past the cache
+    table = ops.rope_table(max_seq + 1, h)
+    out = []
+    for pieces in ((0, rows), (0, 25, rows)):
+        kc = torch.zeros((1, max_seq, kv_heads, h), dtype=torch.float16 if kv == "f16" else torch.int8, device="cuda")
+        vc = torch.zeros_like(kc)
+        ks = torch.zeros((1, max_seq, kv_heads), device="cuda") if kv == "i8" else None
+        vs = torch.zeros_like(ks) if kv == "i8" else None
+        q = [ops.rope_kv_append(dev(qkv[a:b]), heads, kv_heads, h, table, dev(pos[a:b]), kc, vc, ks, vs, one_sequence=True)
+             for a, b in zip(pieces, pieces[1:])]
+        out.append([torch.cat(q), kc, vc] + ([ks, vs] if kv == "i8" else []))
+    assert all(torch.equal(a, b) for a, b in zip(*out))
