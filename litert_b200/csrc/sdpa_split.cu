@@ -7,7 +7,7 @@
 // Bound by the cache's bytes, so the work is cut by bytes: the cached tokens of all (sequence, KV head) pairs form
 // one row of 16-token units and every SM gets an equal piece of it, whatever the lengths are. (A grid of fixed
 // chunks per sequence left some SMs two chunks and others one or none: 16 ragged sequences of up to 8192 tokens,
-// 8 heads x 256, fp16: 23.7 us; equal pieces: 16.8.) A piece that covers parts of several pairs
+// 8 heads x 256, fp16, caches in L2: 23.7 us; equal pieces: 16.8 at the time.) A piece that covers parts of several pairs
 // leaves one partial record (un-normalised output, maximum, sum) per pair; a second kernel merges a pair's records.
 #include <cuda.h>
 #include <math_constants.h>
@@ -45,7 +45,7 @@ struct Split {
   static constexpr int kQBytes = 8 * H * (QF32 ? 4 : 2);    // the query heads of a pair
   static constexpr int kSlotBytes = 2 * kOperandBytes + kQBytes;
   // About 128 KB in flight per SM: with a third 64 KB stage the same launch is 1.1 us slower (17.9 against 16.8 us, 16
-  // ragged sequences of up to 8192 tokens), and HBM needs no more to be busy.
+  // ragged sequences of up to 8192 tokens, caches resident in L2).
   static constexpr int kStagesRaw = 146 * 1024 / kSlotBytes;
   static constexpr int kStages = kStagesRaw > 8 ? 8 : kStagesRaw;
   static constexpr int kChunkElems = 16 / kElem;            // elements of a 16-byte piece
@@ -57,8 +57,10 @@ struct Split {
 struct SplitShared {
   uint64_t full_k[8], full_v[8], empty_k[8], empty_v[8];
   uint64_t p_full[2], p_empty[2];
-  uint2 p[2][8][32];       // softmax weights of a stage, as the B fragments of the second product
+  uint4 p[2][8][32];       // softmax weights of a stage, as the B fragments of the second product: heads, remainders
   float alpha[2][8];       // factor on the earlier stages' output, per head
+  uint4 smag[2][2];        // int8 rows: the eight warps' largest value scales over a stage, as bits
+  float unit_of[2];        // int8 rows: what the stage's weights are multiples of
   float smax[2][8][8];     // the warps' maxima over a stage
   float ssum[8][8];
   int pair_b, pair_kvh, unit, units_cta;
@@ -118,10 +120,19 @@ __device__ __forceinline__ uint32_t half2_bits(float a, float b) {
   const __half2 h = __floats2half2_rn(a, b);
   return *reinterpret_cast<const uint32_t*>(&h);
 }
+// What the fp16 roundings of a and b leave, as fp16.
+__device__ __forceinline__ uint32_t half2_remainder(float a, float b, uint32_t rounded) {
+  const float2 r = __half22float2(*reinterpret_cast<const __half2*>(&rounded));
+  return half2_bits(a - r.x, b - r.y);
+}
 __device__ __forceinline__ uint32_t transpose8x8(uint32_t x) {
   uint32_t y;
   asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(y) : "r"(x));
   return y;
+}
+// Exponent field of a magnitude (sign cleared), such that the field and 254 minus it both name normal numbers.
+__device__ __forceinline__ int magnitude_exponent(uint32_t bits) {
+  return min(max((int)(bits >> 23), 1), 253);
 }
 // Four int8 -> two half2, exactly: bias to unsigned, splice into 1024 + u, subtract 1152.
 __device__ __forceinline__ void widen_s8x4(uint32_t w, uint32_t& lo_bits, uint32_t& hi_bits) {
@@ -182,13 +193,19 @@ struct SplitMaps {
 //  * A QK warp takes 16 tokens of the stage: S^T[token, head] = K . Q^T with the up-to-eight query heads as the
 //    8-wide side of the MMA. The stage's maximum goes through shared memory (one barrier of the QK warps), the
 //    weights leave as the B fragments of the second product (one 8 x 8 transpose each).
+//    One fp16 rounding of a weight costs 2^-12 on average: float16 and float32 rows carry the remainders as a second
+//    fragment (error against 64 bits, 60 draws of 64 to 8192 tokens, fp16: 2.6e-4 -> 2.1e-4, of which 1.7e-4 are the
+//    output's own rounding; +0.4 us at 16 x 8192). int8 rows' weights hold the value scales, which may be far below
+//    fp16's range: they are in units of a power of two next to the largest scale so far (scales of 3e-4: 4.5e-4 ->
+//    2.9e-4; +0.5 us).
 //  * A PV warp takes 64 of the head's dimensions for all tokens of the stage: O^T[d, head] += V^T . P^T, the rows
 //    paired up by byte permutes. So no output has to be merged between warps, and while the PV warps work on a
 //    stage the QK warps are at the next.
-// Measured on B200 with the merge (16 sequences, lengths uniform up to 8192, 8 heads x 256 on one KV head): fp16 rows
-// 23.7 -> 16.8 us (61 MB: 3.6 TB/s; about 6 us are the two kernels' hand-offs, the first copies' latency and the merge),
-// int8 rows 20.6 -> 15.6 (bound by instruction issue: widening the bytes and pairing them up); 4 x 2000 masked float32
-// tokens of two KV heads 13.9 -> 7.7.
+// Measured on B200 with the merge, replayed, against a grid of fixed chunks per sequence (16 sequences, lengths uniform
+// up to 8192, 8 heads x 256 on one KV head; caches resident in L2 / read from HBM): fp16 rows 28.8 / 31.1 -> 15.4 / 19.1 us
+// (61 MB: 3.2 TB/s from HBM; about 6 us are the two kernels' hand-offs, the first copies' latency and the merge), int8 rows
+// 25.3 / 30.8 -> 16.6 / 17.9 (bound by instruction issue: widening the bytes and pairing them up); 4 x 2000 masked float32
+// tokens of two KV heads 13.7 / 16.2 -> 7.7 / 9.1.
 template <int KV, int H, bool QF32>
 __global__ void __launch_bounds__(Split<KV, H, QF32>::kThreads, 1)
     sdpa_split_kernel(const __grid_constant__ SplitMaps maps, const SdpaParams p, const int min_units) {
@@ -370,6 +387,7 @@ __global__ void __launch_bounds__(Split<KV, H, QF32>::kThreads, 1)
         return f;
       };
       float m_run[2] = {-CUDART_INF_F, -CUDART_INF_F}, l_run[2] = {0.0f, 0.0f};
+      uint32_t mag_run = 0;  // int8: the largest value scale so far, as bits
       Factors next = factors(0);
       for (int j = 0; j < seg; j += S::kUnits, ++it) {
         const int s = it % S::kStages;
@@ -432,6 +450,10 @@ __global__ void __launch_bounds__(Split<KV, H, QF32>::kThreads, 1)
           mx[1] = fmaxf(mx[1], __shfl_xor_sync(0xffffffffu, mx[1], o));
         }
         if (g == 0) *reinterpret_cast<float2*>(&sh.smax[pb][w][2 * t]) = make_float2(mx[0], mx[1]);
+        if constexpr (KV == kKvI8) {
+          const uint32_t mag = __reduce_max_sync(0xffffffffu, max(__float_as_uint(fabsf(f.sa)), __float_as_uint(fabsf(f.sb))));
+          if (lane == 0) reinterpret_cast<uint32_t*>(sh.smag[pb])[w] = mag;
+        }
         named_barrier(1, 32 * S::kQkWarps);
         float alpha[2], m_use[2];
 #pragma unroll
@@ -447,16 +469,40 @@ __global__ void __launch_bounds__(Split<KV, H, QF32>::kThreads, 1)
         float pb0 = exp2f(sc[2] - m_use[0]), pb1 = exp2f(sc[3] - m_use[1]);
         l_run[0] = l_run[0] * alpha[0] + (pa0 + pb0);
         l_run[1] = l_run[1] * alpha[1] + (pa1 + pb1);
+        float unit_now = 1.0f;
         if constexpr (KV == kKvI8) {
-          pa0 *= f.sa;
-          pa1 *= f.sa;
-          pb0 *= f.sb;
-          pb1 *= f.sb;
+          static_assert(S::kQkWarps == 8, "two words of four warps");
+          const uint4 m0 = sh.smag[pb][0], m1 = sh.smag[pb][1];
+          const int was = magnitude_exponent(mag_run);
+          mag_run = max(max(max(mag_run, m0.x), max(m0.y, m0.z)), max(max(m0.w, m1.x), max(m1.y, max(m1.z, m1.w))));
+          const int now = magnitude_exponent(mag_run);
+          if (now != was) {  // the earlier stages' outputs are in the smaller unit
+            const float f = exp2f((float)(was - now));
+            alpha[0] *= f;
+            alpha[1] *= f;
+          }
+          unit_now = __int_as_float(now << 23);
+          const float per_unit = __int_as_float((254 - now) << 23);
+          const float sa = f.sa * per_unit, sb = f.sb * per_unit;
+          pa0 *= sa;
+          pa1 *= sa;
+          pb0 *= sb;
+          pb1 *= sb;
         }
         // rows = tokens g (g + 8), columns = heads 2t, 2t + 1 -> head g; tokens 2t, 2t + 1 (2t + 8, 2t + 9)
-        const uint2 frag = make_uint2(transpose8x8(half2_bits(pa0, pa1)), transpose8x8(half2_bits(pb0, pb1)));
+        const uint32_t wa = half2_bits(pa0, pa1), wb = half2_bits(pb0, pb1);
+        uint4 frag = make_uint4(transpose8x8(wa), transpose8x8(wb), 0u, 0u);
+        if constexpr (KV != kKvI8) {
+          frag.z = transpose8x8(half2_remainder(pa0, pa1, wa));
+          frag.w = transpose8x8(half2_remainder(pb0, pb1, wb));
+        }
         mbar_wait_bounded(&sh.p_empty[pb], ((it >> 1) & 1u) ^ 1u, abort_flag, p.status, kStatusWaitTimeoutEmpty);
-        sh.p[pb][w][lane] = frag;
+        if constexpr (KV == kKvI8) {
+          *reinterpret_cast<uint2*>(&sh.p[pb][w][lane]) = make_uint2(frag.x, frag.y);
+          if (w == 0 && lane == 0) sh.unit_of[pb] = unit_now;
+        } else {
+          sh.p[pb][w][lane] = frag;
+        }
         if (w == 0 && g == 0) *reinterpret_cast<float2*>(&sh.alpha[pb][2 * t]) = make_float2(alpha[0], alpha[1]);
         __syncwarp();
         if (lane == 0) mbar_arrive(&sh.p_full[pb]);
@@ -495,9 +541,12 @@ __global__ void __launch_bounds__(Split<KV, H, QF32>::kThreads, 1)
     while (left > 0) {
       const int seg = min(left, units_of(len) - unit);
       const int t_end = min(len, (unit + seg) * kUnit);
-      float o[4][4];
+      float o[4][4], rem[4][4], unit_now = 1.0f;  // rem: what the weights' remainders give (chains of their own)
 #pragma unroll
-      for (int i = 0; i < 4; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.0f;
+      for (int i = 0; i < 4; ++i) {
+        o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.0f;
+        rem[i][0] = rem[i][1] = rem[i][2] = rem[i][3] = 0.0f;
+      }
       for (int j = 0; j < seg; j += S::kUnits, ++it) {
         const int s = it % S::kStages;
         const uint32_t ph = (it / S::kStages) & 1u;
@@ -507,17 +556,30 @@ __global__ void __launch_bounds__(Split<KV, H, QF32>::kThreads, 1)
         mbar_wait_bounded(&sh.full_v[s], ph, abort_flag, p.status, kStatusWaitTimeoutFull);
         mbar_wait_bounded(&sh.p_full[pb], (it >> 1) & 1u, abort_flag, p.status, kStatusWaitTimeoutFull);
         const float2 al = *reinterpret_cast<const float2*>(&sh.alpha[pb][2 * t]);
+        if constexpr (KV == kKvI8) unit_now = sh.unit_of[pb];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           o[i][0] *= al.x;
           o[i][1] *= al.y;
           o[i][2] *= al.x;
           o[i][3] *= al.y;
+          if constexpr (KV != kKvI8) {
+            rem[i][0] *= al.x;
+            rem[i][1] *= al.y;
+            rem[i][2] *= al.x;
+            rem[i][3] *= al.y;
+          }
         }
         const uint32_t vbase = ring_a + (uint32_t)(s * 2 + 1) * S::kOperandBytes;
 #pragma unroll 4
         for (int k = 0; k < n; ++k) {
-          const uint2 pf = sh.p[pb][k][lane];
+          uint4 pf;
+          if constexpr (KV == kKvI8) {
+            const uint2 v = *reinterpret_cast<const uint2*>(&sh.p[pb][k][lane]);
+            pf = make_uint4(v.x, v.y, 0u, 0u);
+          } else {
+            pf = sh.p[pb][k][lane];
+          }
           const uint32_t ubase = vbase + (uint32_t)k * S::kUnitBytes;
           const int last_row = last - k * kUnit;
           uint32_t vr[4][4];  // 8 head dimensions of tokens 2t, 2t + 1, 2t + 8, 2t + 9
@@ -543,9 +605,12 @@ __global__ void __launch_bounds__(Split<KV, H, QF32>::kThreads, 1)
             }
           }
 #pragma unroll
-          for (int i = 0; i < 4; ++i)  // MMA row g <-> the thread's dimension 2 i, row g + 8 <-> 2 i + 1
-            mma_f16(o[i], __byte_perm(vr[0][i], vr[1][i], 0x5410), __byte_perm(vr[0][i], vr[1][i], 0x7632),
-                    __byte_perm(vr[2][i], vr[3][i], 0x5410), __byte_perm(vr[2][i], vr[3][i], 0x7632), pf.x, pf.y);
+          for (int i = 0; i < 4; ++i) {  // MMA row g <-> the thread's dimension 2 i, row g + 8 <-> 2 i + 1
+            const uint32_t a0 = __byte_perm(vr[0][i], vr[1][i], 0x5410), a1 = __byte_perm(vr[0][i], vr[1][i], 0x7632);
+            const uint32_t a2 = __byte_perm(vr[2][i], vr[3][i], 0x5410), a3 = __byte_perm(vr[2][i], vr[3][i], 0x7632);
+            mma_f16(o[i], a0, a1, a2, a3, pf.x, pf.y);
+            if constexpr (KV != kKvI8) mma_f16(rem[i], a0, a1, a2, a3, pf.z, pf.w);
+          }
         }
         __syncwarp();
         if (lane == 0) {
@@ -553,6 +618,10 @@ __global__ void __launch_bounds__(Split<KV, H, QF32>::kThreads, 1)
           mbar_arrive(&sh.p_empty[pb]);
         }
       }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[i][e] = KV == kKvI8 ? o[i][e] * unit_now : o[i][e] + rem[i][e];
       float* rec = p.ws + ((size_t)blockIdx.x + (size_t)b * p.nkv + kvh) * 8 * S::kRec;
 #pragma unroll
       for (int e = 0; e < 2; ++e) {

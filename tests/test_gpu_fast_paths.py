@@ -180,3 +180,59 @@ def test_rotation_of_many_rows_equals_that_of_a_few(ops, kv, heads, kv_heads, h)
              for a, b in zip(pieces, pieces[1:])]
         out.append([torch.cat(q), kc, vc] + ([ks, vs] if kv == "i8" else []))
     assert all(torch.equal(a, b) for a, b in zip(*out))
+
+
+def _decode_case(rng, lengths, s_max, n, nkv, h):
+    """Queries that fp16 holds exactly, int8 keys with scales: the logits of float32 arithmetic over exact operands."""
+    b = len(lengths)
+    q = rng.standard_normal((b, 1, n, h)).astype(np.float16).astype(np.float32)
+    k8 = rng.integers(-127, 128, (b, s_max, nkv, h)).astype(np.int8)
+    ks = rng.uniform(0.005, 0.02, (b, s_max, nkv)).astype(np.float32)
+    return q, k8, ks
+
+
+@pytest.mark.parametrize("scales", ["small", "growing", "shrinking", "zeros among them", "large"])
+@pytest.mark.parametrize("n,nkv,h", [(8, 1, 256), (6, 2, 128), (4, 4, 64)])
+def test_sdpa_decode_int8_value_scales_of_any_size(ops, ws, scales, n, nkv, h):
+    """Softmax weights times value scales are fp16 operands: scales far below and above what fp16 holds, and such that
+    change along the cache, cost no more than those near one. Bound: an fp16 rounding (2^-11) of each weight, and half
+    the smallest fp16 step (2^-25) of the largest scale, which is counted in units of at most twice itself."""
+    rng = np.random.default_rng(h)
+    s_max, lengths = 1500, np.asarray([1500, 0, 700, 33, 1], np.int32)
+    b = len(lengths)
+    q, k8, ks = _decode_case(rng, lengths, s_max, n, nkv, h)
+    v8 = rng.integers(-127, 128, (b, s_max, nkv, h)).astype(np.int8)
+    vs = rng.uniform(0.5, 1.0, (b, s_max, nkv))
+    steps = np.linspace(-9, 3, s_max)[None, :, None]
+    vs = {"small": vs * 1e-6, "growing": vs * 10.0 ** steps, "shrinking": vs * 10.0 ** -steps,
+          "zeros among them": vs * 1e-4 * (rng.random(vs.shape) < 0.5), "large": vs * 1e6}[scales].astype(np.float32)
+    out = ops.sdpa_decode(dev(q), dev(k8), dev(v8), lengths=dev(lengths), k_scale=dev(ks), v_scale=dev(vs), ws=ws)
+    out = out.cpu().numpy()
+    kf, vf = k8.astype(np.float64) * ks[..., None], v8.astype(np.float64) * vs[..., None]
+    for i, length in enumerate(lengths):
+        if length == 0:
+            assert not out[i].any()
+            continue
+        want = _attention(q[i, 0], kf[i], vf[i], int(length), 1.0 / np.sqrt(h), 0.0)
+        size = _attention(q[i, 0], kf[i], np.abs(vf[i]), int(length), 1.0 / np.sqrt(h), 0.0)
+        top = np.repeat(vs[i, :length].max(0), n // nkv)[:, None] * 127.0
+        assert np.all(np.abs(out[i, 0] - want) <= 1.05 * 2.0 ** -11 * size + 2.0 ** -24 * top), i
+
+
+@pytest.mark.parametrize("kv", ["f16", "f32"])
+@pytest.mark.parametrize("n,nkv,h", [(8, 1, 256), (6, 2, 128), (4, 4, 64)])
+def test_sdpa_decode_weights_are_not_rounded_to_fp16(ops, ws, kv, n, nkv, h):
+    """float16 and float32 rows: a weight is the sum of two fp16 operands (2^-22 of it is lost), so that with operands
+    fp16 holds and float32 outputs only float32 arithmetic is left: 2h products per logit of a few units at 2^-23
+    each, taken as 2^-15 of the output. A single fp16 weight is 2^-12 off, 1.8e-4 here."""
+    rng = np.random.default_rng(h)
+    s_max, lengths = 900, np.asarray([900, 64, 333], np.int32)
+    b = len(lengths)
+    half = lambda a: a.astype(np.float16).astype(np.float32)
+    q = half(rng.standard_normal((b, 1, n, h)))
+    k, v = half(rng.standard_normal((b, s_max, nkv, h))), half(rng.standard_normal((b, s_max, nkv, h)))
+    t = np.float16 if kv == "f16" else np.float32
+    out = ops.sdpa_decode(dev(q), dev(k.astype(t)), dev(v.astype(t)), lengths=dev(lengths), ws=ws).cpu().numpy()
+    for i, length in enumerate(lengths):
+        want = _attention(q[i, 0], k[i], v[i], int(length), 1.0 / np.sqrt(h), 0.0)
+        assert np.linalg.norm(out[i, 0] - want) <= 2.0 ** -15 * np.linalg.norm(want), i
