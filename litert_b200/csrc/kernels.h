@@ -160,6 +160,7 @@ struct SdpaParams {
   int m_alloc;
   size_t ws_bytes;
   int* status;
+  int expired;   // 1: every device-side wait counts as run out (tests of what the caller then sees)
   // > 1: rows b * rows_per_kv .. + rows_per_kv - 1 are the query tokens of sequence b and attend over
   // that sequence's cache (the composite with several query tokens; q / out / mask are then indexed by row)
   int rows_per_kv;
@@ -191,6 +192,8 @@ struct AttnStepParams {
 bool attn_step_supported(int n, int nkv, int h, int kv_dtype);
 cudaError_t launch_attn_step(const AttnStepParams& p, cudaStream_t s);
 cudaError_t launch_sdpa_decode(const SdpaParams& p, cudaStream_t s);
+// What SdpaParams::expired is for launches of the calling thread: 0, or what b200_test_expire_waits set.
+int& expired_waits();
 size_t sdpa_workspace_bytes(int b, int n, int nkv, int h, int s_max, int shared_kv = 0);
 size_t sdpa_chunk_workspace_bytes(int b, int nkv, int h, int s_max, int shared_kv = 0);
 // One query row per sequence (sdpa_split.cu): the ragged decode step.

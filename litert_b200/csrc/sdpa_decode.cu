@@ -472,7 +472,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) sdpa_rows_mma_kernel(const Sdp
   if (tid == 0) {
     mbar_init(&bar[0], 1);
     mbar_init(&bar[1], 1);
-    s_abort = 0;
+    s_abort = p.expired;
     mbar_fence_init();
   }
   pdl_enter();
@@ -499,7 +499,10 @@ __global__ void __launch_bounds__(kWarps * 32, 2) sdpa_rows_mma_kernel(const Sdp
   const uint8_t* src = static_cast<const uint8_t*>(warp < 2 ? p.k : p.v) + (size_t)kvh * L::kRaw;
   uint8_t* dst = rsmem + (warp < 2 ? L::kKOff : L::kVOff) + (size_t)(tid & 63) * L::kRawPitch;
   auto tile_first = [&](int j) { return c0 + (j + (int)blockIdx.z) % tiles * kRowsTile; };
+  int armed = 0;  // fetches of this thread's half
   auto fetch = [&](int j, int which) {  // (the threads of that half; a phase stays open until its bytes are announced)
+    if (*abort_flag) return;  // a barrier must not be armed twice in a phase, and after an abort its wait says nothing
+    ++armed;
     if (tid == which * 64) mbar_arrive_expect_tx(&bar[which], (uint32_t)(kRowsTile * L::kRaw));
     bulk_g2s(dst, src + (size_t)min(tile_first(j) + (tid & 63), c1 - 1) * pitch, L::kRaw, &bar[which]);
   };
@@ -729,10 +732,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) sdpa_rows_mma_kernel(const Sdp
     if constexpr (KV == kKvF16)
       if (warp >= 2 && j + 1 < tiles) fetch(j + 1, 1);
   }
-  if (__syncthreads_or(*abort_flag)) {  // never leave with copies in flight
-    mbar_drain_bounded(&bar[0], (uint32_t)(tiles - 1) & 1u);
-    mbar_drain_bounded(&bar[1], (uint32_t)(tiles - 1) & 1u);
-  }
+  if (__syncthreads_or(*abort_flag) && armed > 0) mbar_drain_bounded(&bar[warp >> 1], (uint32_t)(armed - 1) & 1u);  // copies in flight
 #pragma unroll
   for (int e = 0; e < 2; ++e) {
     l_run[e] += __shfl_xor_sync(0xffffffffu, l_run[e], 1);
@@ -1481,7 +1481,14 @@ size_t sdpa_workspace_bytes(int b, int n, int nkv, int h, int s_max, int shared_
   return shared_kv ? chunks : std::max(chunks, sdpa_split_workspace_bytes(b, nkv, h, s_max));
 }
 
-cudaError_t launch_sdpa_decode(const SdpaParams& p, cudaStream_t s) {
+int& expired_waits() {
+  static thread_local int v = 0;
+  return v;
+}
+
+cudaError_t launch_sdpa_decode(const SdpaParams& given, cudaStream_t s) {
+  SdpaParams p = given;
+  p.expired = expired_waits();
   if (sdpa_split_supported(p)) return launch_sdpa_split(p, s);
   const bool qf32 = p.q_dtype == 1;
   switch (p.kv_dtype) {

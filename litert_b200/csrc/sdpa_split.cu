@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(Split<KV, H, QF32>::kThreads, 1)
       mbar_init(&sh.p_full[i], S::kQkWarps);
       mbar_init(&sh.p_empty[i], S::kPvWarps);
     }
-    sh.abort_flag = 0;
+    sh.abort_flag = p.expired;
     mbar_fence_init();
     for (int op = 0; op < 2; ++op) {
       asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.stage[op]) : "memory");
@@ -295,10 +295,12 @@ __global__ void __launch_bounds__(Split<KV, H, QF32>::kThreads, 1)
   if (warp == 0) {
     // ---------------- producer ----------------
     if (lane == 0) {
-      while (left > 0) {
+      uint32_t armed[2] = {0, 0};  // copies of keys and values
+      bool stop = false;
+      while (left > 0 && !stop) {
         const int seg = min(left, units_of(len) - unit);
         const int row0 = (p.rows_per_kv > 1 ? b / p.rows_per_kv : b) * p.s_max;
-        for (int j = 0; j < seg; j += S::kUnits, ++it) {
+        for (int j = 0; j < seg && !stop; j += S::kUnits, ++it) {
           const int s = it % S::kStages;
           const uint32_t ph = (it / S::kStages) & 1u;
           const int n = min(S::kUnits, seg - j);
@@ -307,9 +309,14 @@ __global__ void __launch_bounds__(Split<KV, H, QF32>::kThreads, 1)
           for (int op = 0; op < 2; ++op) {
             uint64_t* full = op ? &sh.full_v[s] : &sh.full_k[s];
             mbar_wait_bounded(op ? &sh.empty_v[s] : &sh.empty_k[s], ph ^ 1u, abort_flag, p.status, kStatusWaitTimeoutEmpty);
+            // After an abort that wait says nothing: the slot's last copy may be in flight, and a barrier must not be
+            // armed twice in a phase.
+            stop = *abort_flag != 0;
+            if (stop) break;
             const bool with_q = op == 0 && j == 0;  // the segment's queries come with its first keys
             const uint32_t q_bytes = (uint32_t)(group * H * (QF32 ? 4 : 2));
             mbar_arrive_expect_tx(full, (uint32_t)(n * kUnit * S::kRowBytes) + (with_q ? q_bytes : 0u));
+            ++armed[op];
             if (with_q)
               bulk_g2s_at(q_smem + (uint32_t)s * S::kQBytes,
                           static_cast<const uint8_t*>(p.q) + ((size_t)b * p.n + kvh * group) * H * (QF32 ? 4 : 2), q_bytes, full);
@@ -326,11 +333,12 @@ __global__ void __launch_bounds__(Split<KV, H, QF32>::kThreads, 1)
         if (left > 0) next_pair();
       }
       // never leave with copies in flight (only possible after an abort)
-      for (uint32_t back = 0; back < (uint32_t)S::kStages && back < it; ++back) {
-        const uint32_t j = it - 1 - back;
-        mbar_drain_bounded(&sh.full_k[j % S::kStages], (j / S::kStages) & 1u);
-        mbar_drain_bounded(&sh.full_v[j % S::kStages], (j / S::kStages) & 1u);
-      }
+#pragma unroll 1
+      for (int op = 0; op < 2; ++op)
+        for (uint32_t back = 0; back < (uint32_t)S::kStages && back < armed[op]; ++back) {
+          const uint32_t j = armed[op] - 1 - back;
+          mbar_drain_bounded(op ? &sh.full_v[j % S::kStages] : &sh.full_k[j % S::kStages], (j / S::kStages) & 1u);
+        }
     }
   } else if (warp <= S::kQkWarps) {
     // ---------------- first product and softmax ----------------

@@ -395,4 +395,8 @@ int b200_sdpa_rows(const void* d_q, const void* d_k, const void* d_v, const floa
   return e == cudaSuccess ? B200_OK : cuda_fail(e, "b200_sdpa_rows");
 }
 
+// For tests, not in the header: from now on (0: until now) every device-side wait of this thread's attention calls counts
+// as run out.
+B200_API void b200_test_expire_waits(int on) { b200::expired_waits() = on; }
+
 }  // extern "C"
