@@ -114,6 +114,15 @@ __device__ __forceinline__ void mbar_wait_bounded(uint64_t* bar, uint32_t parity
   if (status) atomicCAS(status, 0, code);  // (entry points without a status word still end in bounded time)
 }
 
+// Attention over pieces: the denominator in a record whose CTA gave up on a wait. A merge that meets one answers NaN for
+// the head, so that a caller without a status word is not handed plausible numbers.
+constexpr float kLostRecord = -1.0f;
+// A head's output from its summed records: no cached token (or every key masked out) gives zero, not 0 / 0.
+__device__ __forceinline__ float head_output(float acc, float denominator) {
+  if (denominator > 0.0f) return acc / denominator;
+  return denominator == kLostRecord ? __int_as_float(0x7fffffff) : 0.0f;
+}
+
 // Last resort after an abort: waits (10 ms at most, whatever the abort flag says) for a copy that was
 // issued towards `bar`, so that a CTA does not exit with copies into its shared memory in flight.
 __device__ __forceinline__ void mbar_drain_bounded(uint64_t* bar, uint32_t parity) {

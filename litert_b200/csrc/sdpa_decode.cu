@@ -732,7 +732,8 @@ __global__ void __launch_bounds__(kWarps * 32, 2) sdpa_rows_mma_kernel(const Sdp
     if constexpr (KV == kKvF16)
       if (warp >= 2 && j + 1 < tiles) fetch(j + 1, 1);
   }
-  if (__syncthreads_or(*abort_flag) && armed > 0) mbar_drain_bounded(&bar[warp >> 1], (uint32_t)(armed - 1) & 1u);  // copies in flight
+  const bool lost = __syncthreads_or(*abort_flag) != 0;
+  if (lost && armed > 0) mbar_drain_bounded(&bar[warp >> 1], (uint32_t)(armed - 1) & 1u);  // copies in flight
 #pragma unroll
   for (int e = 0; e < 2; ++e) {
     l_run[e] += __shfl_xor_sync(0xffffffffu, l_run[e], 1);
@@ -747,7 +748,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) sdpa_rows_mma_kernel(const Sdp
     for (int i = 0; i < H / 8; ++i) *reinterpret_cast<float2*>(rec + i * 8 + 2 * t) = make_float2(o[i][2 * e], o[i][2 * e + 1]);
     if (t == 0) {
       rec[H] = m_run[e];
-      rec[H + 1] = l_run[e];
+      rec[H + 1] = lost ? kLostRecord : l_run[e];
     }
   }
 }
@@ -1177,14 +1178,17 @@ __global__ void sdpa_merge_kernel(const SdpaParams p, const int chunk_tokens, co
     for (int o = 16; o > 0; o >>= 1) mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, o));
     const float muse = mm == -CUDART_INF_F ? 0.0f : mm;
     float l = 0.0f;
+    bool lost = false;
     for (int c = lane; c < chunks; c += 32) {
-      const float f = exp2f(base[c * cstride + H] - muse);
+      const float f = exp2f(base[c * cstride + H] - muse), sum = base[c * cstride + H + 1];
       merge_w[c] = f;
-      l += f * base[c * cstride + H + 1];
+      l += f * sum;
+      lost = lost || sum == kLostRecord;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-    if (lane == 0) s_l = l;
+    lost = __any_sync(0xffffffffu, lost);
+    if (lane == 0) s_l = lost ? kLostRecord : l;
   }
   __syncthreads();
   float acc = 0.0f;
@@ -1200,8 +1204,7 @@ __global__ void sdpa_merge_kernel(const SdpaParams p, const int chunk_tokens, co
     for (int j = 0; j < 8; ++j)
       if (c + j < chunks) acc += merge_w[c + j] * v[j];
   }
-  const float l = s_l;
-  const float out = l > 0.0f ? acc / l : 0.0f;  // no cached token (or every key masked out): zeros, not 0 / 0
+  const float out = head_output(acc, s_l);
   const size_t oi = ((size_t)b * p.n + head) * H + d;
   if constexpr (QF32) {
     static_cast<float*>(p.out)[oi] = out;

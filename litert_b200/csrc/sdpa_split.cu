@@ -645,6 +645,16 @@ __global__ void __launch_bounds__(Split<KV, H, QF32>::kThreads, 1)
       if (left > 0) next_pair();
     }
   }
+  if (!__syncthreads_or(*abort_flag)) return;
+  // the records are made of whatever the ring held
+  left = sh.units_cta, b = sh.pair_b, kvh = sh.pair_kvh, unit = sh.unit;
+  len = row_length(p, b);
+  while (left > 0) {
+    const int seg = min(left, units_of(len) - unit);
+    if (tid < 8) p.ws[((size_t)blockIdx.x + (size_t)b * p.nkv + kvh) * 8 * S::kRec + tid * S::kRec + H + 1] = kLostRecord;
+    left -= seg;
+    if (left > 0) next_pair();
+  }
 }
 
 // Records of one (row, KV head) pair: the first one, and how many.
@@ -664,7 +674,7 @@ __device__ __forceinline__ PairRecords pair_records(const SdpaParams& p, int b, 
 }
 
 // Weights exp2(m_record - m) of a head's records, from their (maximum, sum) pairs at `ml`; returns the softmax
-// denominator. Whole warp; the first 64 pairs in one round trip.
+// denominator, or kLostRecord where a record is one. Whole warp; the first 64 pairs in one round trip.
 __device__ __forceinline__ float record_weights(const float* ml, size_t stride, int count, int lane, float* weights) {
   const float2 none = make_float2(-CUDART_INF_F, 0.0f);
   const float2 a = lane < count ? __ldcg(reinterpret_cast<const float2*>(ml + lane * stride)) : none;
@@ -676,6 +686,7 @@ __device__ __forceinline__ float record_weights(const float* ml, size_t stride, 
   const float muse = mm == -CUDART_INF_F ? 0.0f : mm;
   const float fa = exp2f(a.x - muse), fb = exp2f(b.x - muse);
   float l = fa * a.y + fb * b.y;
+  bool lost = a.y == kLostRecord || b.y == kLostRecord;
   if (lane < count) weights[lane] = fa;
   if (lane + 32 < count) weights[lane + 32] = fb;
   for (int c = lane + 64; c < count; c += 32) {
@@ -683,10 +694,11 @@ __device__ __forceinline__ float record_weights(const float* ml, size_t stride, 
     const float f = exp2f(v.x - muse);
     weights[c] = f;
     l += f * v.y;
+    lost = lost || v.y == kLostRecord;
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-  return l;
+  return __any_sync(0xffffffffu, lost) ? kLostRecord : l;
 }
 
 // Sum of a head's records, weighted, for the four outputs d4 .. d4 + 3: records grp, grp + groups, ...
@@ -768,8 +780,8 @@ __global__ void __launch_bounds__(kMergeThreads) sdpa_split_merge_kernel(const S
     acc.z += v.z;
     acc.w += v.w;
   }
-  const float l = s_l;  // no cached token (or every key masked out): zeros, not 0 / 0
-  acc = l > 0.0f ? make_float4(acc.x / l, acc.y / l, acc.z / l, acc.w / l) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  const float l = s_l;
+  acc = make_float4(head_output(acc.x, l), head_output(acc.y, l), head_output(acc.z, l), head_output(acc.w, l));
   const size_t oi = ((size_t)b * p.n + head) * H + 4 * quad;
   if constexpr (QF32) {
     float* o = static_cast<float*>(p.out) + oi;
@@ -818,18 +830,20 @@ __global__ void __launch_bounds__(kMergeQuantThreads, 2) sdpa_split_merge_quant_
     if (quad < quads) base[e] = quad_base(quad, &count[e]);
     request_quads(first[e], base[e], kStride, count[e], 0, 1);
   }
+  bool lost = false;
   for (int hd = threadIdx.x >> 5; hd < p.n; hd += blockDim.x >> 5) {
     const PairRecords r = pair_records<H>(p, b, hd / group, units, below, cut);
     const float l = record_weights(r.first + (hd % group) * kRec + H, kStride, r.count, lane, wts + hd * split_ctas);
     if (lane == 0) s_l[hd & 63] = l;
+    lost = lost || l == kLostRecord;
   }
-  __syncthreads();
+  lost = __syncthreads_or(lost) != 0;
   float mn = 3.402823466e+38f, mx = -3.402823466e+38f;
   auto finish = [&](int quad, const float* from, int n, const float4 (&requested)[kMergeBatch]) {
     const int head = quad * 4 / H;
     float4 acc = merge_quad(from, kStride, n, 0, 1, wts + head * split_ctas, requested);
     const float l = s_l[head & 63];  // an empty sequence gives a zero row
-    acc = l > 0.0f ? make_float4(acc.x / l, acc.y / l, acc.z / l, acc.w / l) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    acc = make_float4(head_output(acc.x, l), head_output(acc.y, l), head_output(acc.z, l), head_output(acc.w, l));
     *reinterpret_cast<float4*>(xs + 4 * quad) = acc;
     if (p.out) {
       float* o = static_cast<float*>(p.out) + (size_t)b * width + 4 * quad;
@@ -849,6 +863,7 @@ __global__ void __launch_bounds__(kMergeQuantThreads, 2) sdpa_split_merge_quant_
   }
   const int k_pad = (width + 127) / 128 * 128;
   quantize_smem_row(xs, width, k_pad, b, p.m_alloc, mn, mx, p.q_tiled_out, p.out_scales, p.out_zps, red);
+  if (lost && threadIdx.x == 0) p.out_scales[b] = __int_as_float(0x7fffffff);  // (integers hold no NaN; their scale does)
 }
 
 // Shortest piece worth a CTA of its own.

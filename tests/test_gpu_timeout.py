@@ -141,7 +141,8 @@ def _attention_inputs(kv, b, s, n, nkv, h):
 @pytest.mark.parametrize("n,nkv,h", [(8, 1, 256), (6, 2, 128), (4, 4, 64)])
 def test_attention_whose_waits_run_out_ends_and_the_next_call_is_right(expire_waits, kv, n, nkv, h):
     """The kernels' loops go on after a wait that ran out, without another copy (a barrier armed twice in a phase has no
-    defined state), and end; what runs next is not affected."""
+    defined state), and end; what runs next is not affected. The result is NaN where there was anything to attend to:
+    these entry points have no status word to look at."""
     from litert_b200 import ops
 
     q, k, v, kw = _attention_inputs(kv, 3, 1000, n, nkv, h)
@@ -156,8 +157,25 @@ def test_attention_whose_waits_run_out_ends_and_the_next_call_is_right(expire_wa
         torch.cuda.synchronize()
         expire_waits(1)
         t0 = time.perf_counter()
-        call()
+        got = call()
         torch.cuda.synchronize()
         assert time.perf_counter() - t0 < 1.0
         expire_waits(0)
+        if kv != "f32" or call is calls[0]:  # (float32 rows of a prompt are loaded without a wait)
+            attended = want.abs().amax(-1) > 0
+            assert torch.isnan(got[attended]).all() and not got[~attended].any()
         assert torch.equal(call(), want)
+
+
+def test_quantized_attention_whose_waits_run_out_gives_a_scale_that_is_not_a_number(expire_waits):
+    from litert_b200 import ops
+
+    q, k, v, kw = _attention_inputs("i8", 2, 500, 8, 1, 128)
+    lengths = torch.tensor([500, 0], dtype=torch.int32, device="cuda")
+    call = lambda: ops.sdpa_decode_quantized(q, k, v, lengths, **kw)
+    want = call()
+    expire_waits(1)
+    got = call().scales[:2]
+    expire_waits(0)
+    assert torch.isnan(got[0]) and got[1] == 1.0
+    assert torch.equal(call().scales[:2], want.scales[:2])
