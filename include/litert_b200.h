@@ -157,7 +157,12 @@ B200_API int b200_fc_w4(const float* d_x, int m, int k, const void* d_w4_packed,
  * per sequence; d_mask [b,1,1,s_max] (optional) is the reference's additive
  * mask. scale <= 0 means 1/sqrt(h) (sdpa.cc:99-105). logit_cap > 0 applies
  * cap*tanh(x/cap) before the mask
- * (tflite/delegates/xnnpack/xnnpack_delegate.cc:6639-6678). */
+ * (tflite/delegates/xnnpack/xnnpack_delegate.cc:6639-6678).
+ * Head sizes 64, 128 and 256 with at most 8 query heads per KV head run on the
+ * fast kernels when q and k / v lie on 16-byte boundaries (int8 caches: 8 is
+ * enough, 16 is faster); anything else runs on a fallback that holds the logits
+ * in shared memory (s_max + h <= 51200, else B200_ERR_UNSUPPORTED). The
+ * workspace may lie anywhere. */
 B200_API size_t b200_sdpa_workspace_bytes(int b, int n, int nkv, int h, int s_max);
 B200_API int b200_sdpa_decode(const void* d_q, const void* d_k, const void* d_v, const float* d_k_scale,
                               const float* d_v_scale, const int32_t* d_lengths, const float* d_mask,

@@ -195,6 +195,9 @@ cudaError_t launch_sdpa_decode(const SdpaParams& p, cudaStream_t s);
 // What SdpaParams::expired is for launches of the calling thread: 0, or what b200_test_expire_waits set.
 int& expired_waits();
 size_t sdpa_workspace_bytes(int b, int n, int nkv, int h, int s_max, int shared_kv = 0);
+// Whether the fallback takes a call (head layouts, sizes or alignments that no other kernel does): its logits must fit
+// in shared memory.
+bool sdpa_runs_generic(const SdpaParams& p);
 size_t sdpa_chunk_workspace_bytes(int b, int nkv, int h, int s_max, int shared_kv = 0);
 // One query row per sequence (sdpa_split.cu): the ragged decode step.
 bool sdpa_split_supported(const SdpaParams& p);

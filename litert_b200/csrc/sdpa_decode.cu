@@ -356,6 +356,74 @@ struct WarpAttention {
   }
 };
 
+// One query row per sequence, the cache cut into chunks of fixed length, rows straight from global memory into MMA
+// fragments.
+template <int KV, int H, bool QF32, int GPI>
+__global__ void __launch_bounds__(kWarps * 32) sdpa_decode_kernel(const SdpaParams p, const int chunk_tokens,
+                                                                  const int chunks_max) {
+  using WA = WarpAttention<KV, H, GPI>;
+  constexpr int KSTEPS = WA::KSTEPS;
+  pdl_enter();
+  const int b = blockIdx.z, kvh = blockIdx.y, chunk = blockIdx.x;
+  const int len = p.lengths ? max(0, min(p.lengths[b], p.s_max)) : p.s_max;
+  const int c0 = chunk * chunk_tokens;
+  if (c0 >= len) return;
+  const int c1 = min(len, c0 + chunk_tokens);
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int g = lane >> 2, t = lane & 3;
+  const int group = p.n / p.nkv;  // query heads per kv head (<= 8)
+
+  // ---- Q fragments: thread (g,t) keeps head g, 16-byte pieces t + 4 i ----
+  uint32_t qf[KSTEPS][4];
+  {
+    const bool head_ok = g < group;
+    const int head = kvh * group + (head_ok ? g : 0);
+#pragma unroll
+    for (int i = 0; i < KSTEPS; ++i) {
+      const int d0 = 8 * (t + 4 * i);
+      if (!head_ok) {
+        qf[i][0] = qf[i][1] = qf[i][2] = qf[i][3] = 0u;
+      } else if constexpr (QF32) {
+        const float* q = static_cast<const float*>(p.q) + ((size_t)b * p.n + head) * H + d0;
+        load8<kKvF32>(q, 0, true, qf[i]);
+      } else {
+        const __half* q = static_cast<const __half*>(p.q) + ((size_t)b * p.n + head) * H + d0;
+        load8<kKvF16>(q, 0, true, qf[i]);
+      }
+    }
+  }
+  WA wa;
+  wa.template run<kSrcGlobal>(p, qf, WA::cache_rows(p, b, kvh), b, c0 + warp * WA::kTokensPerWarpIter, kWarps * WA::kTokensPerWarpIter, c1, lane);
+
+  // ---- merge the warps of this CTA ----
+  __shared__ float sm_m[kWarps][8], sm_l[kWarps][8];
+  __shared__ float sm_o[kWarps][8][H + 4];
+  wa.park(sm_m, sm_l, sm_o, warp, lane);
+  __syncthreads();
+  float* part = p.ws + ((((size_t)b * p.nkv + kvh) * chunks_max + chunk) * 8) * partial_stride(H);
+  for (int idx = tid; idx < group * H; idx += kWarps * 32) {
+    const int head = idx / H, d = idx % H;
+    float mm = -CUDART_INF_F;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) mm = fmaxf(mm, sm_m[w][head]);
+    const float muse = mm == -CUDART_INF_F ? 0.0f : mm;
+    float acc = 0.0f, l = 0.0f;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) {
+      const float f = exp2f(sm_m[w][head] - muse);
+      acc += f * sm_o[w][head][d];
+      l += f * sm_l[w][head];
+    }
+    float* rec = part + (size_t)head * partial_stride(H);
+    rec[d] = acc;
+    if (d == 0) {
+      rec[H] = mm;
+      rec[H + 1] = l;
+    }
+  }
+}
+
 // Prompt-pass variant (SdpaParams::shared_kv): the rows of the batch are consecutive tokens of ONE
 // sequence and all read the same cache, row b up to lengths[b]. Here a WARP owns a row: the warps of a
 // CTA walk the same chunk of the cache for kWarps neighbouring rows at nearly the same pace, so the
@@ -1355,6 +1423,35 @@ int pick_chunk_tokens(int b, int s_max, int shared_kv) {
   return 512;
 }
 
+// The merge behind every kernel that leaves a record per chunk.
+template <int H, bool QF32>
+cudaError_t launch_merge(const SdpaParams& p, int chunk_tokens, int chunks_max, cudaStream_t s) {
+  if (p.q_tiled_out) {
+    if (p.n > 64) return cudaErrorInvalidValue;
+    const size_t smem = sizeof(float) * (size_t)p.n * H;
+    if (smem > 48 * 1024) {
+      cudaError_t ea = cudaFuncSetAttribute(sdpa_merge_quant_kernel<H>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (ea != cudaSuccess) return ea;
+    }
+    // a few rows (a decode step): the widest block per row; many rows (a prompt chunk): several rows per SM
+    return launch_chained(sdpa_merge_quant_kernel<H>, dim3(p.b), dim3(p.b > 32 ? 256 : 1024), smem, s, p, chunk_tokens, chunks_max);
+  }
+  return launch_chained(sdpa_merge_kernel<H, QF32>, dim3(p.n, p.b), dim3(H), sizeof(float) * (size_t)chunks_max, s, p,
+                        chunk_tokens, chunks_max);
+}
+
+template <int KV, int H, bool QF32>
+cudaError_t launch_chunks(const SdpaParams& p, cudaStream_t s) {
+  const int chunk_tokens = pick_chunk_tokens(p.b, p.s_max, 0);
+  const int chunks_max = (p.s_max + chunk_tokens - 1) / chunk_tokens;
+  const dim3 grid(chunks_max, p.nkv, p.b);
+  auto kernel = chunk_tokens == 64    ? sdpa_decode_kernel<KV, H, QF32, 1>
+                : chunk_tokens == 128 ? sdpa_decode_kernel<KV, H, QF32, 2>
+                                      : sdpa_decode_kernel<KV, H, QF32, 4>;
+  const cudaError_t e = launch_chained(kernel, grid, dim3(kWarps * 32), 0, s, p, chunk_tokens, chunks_max);
+  return e == cudaSuccess ? launch_merge<H, QF32>(p, chunk_tokens, chunks_max, s) : e;
+}
+
 template <int KV, int H, bool QF32>
 cudaError_t launch_rows(const SdpaParams& p, cudaStream_t s) {
   int chunk_tokens = pick_chunk_tokens(p.b, p.s_max, p.shared_kv);
@@ -1407,30 +1504,31 @@ cudaError_t launch_rows(const SdpaParams& p, cudaStream_t s) {
     }
   }
   if (e != cudaSuccess) return e;
-  if (p.q_tiled_out) {
-    if (p.n > 64) return cudaErrorInvalidValue;
-    const size_t smem = sizeof(float) * (size_t)p.n * H;
-    if (smem > 48 * 1024) {
-      cudaError_t ea = cudaFuncSetAttribute(sdpa_merge_quant_kernel<H>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (ea != cudaSuccess) return ea;
-    }
-    // a few rows (a decode step): the widest block per row; many rows (a prompt chunk): several rows per SM
-    return launch_chained(sdpa_merge_quant_kernel<H>, dim3(p.b), dim3(p.b > 32 ? 256 : 1024), smem, s, p, chunk_tokens, chunks_max);
-  }
-  return launch_chained(sdpa_merge_kernel<H, QF32>, dim3(p.n, p.b), dim3(H), sizeof(float) * (size_t)chunks_max, s, p,
-                        chunk_tokens, chunks_max);
+  return launch_merge<H, QF32>(p, chunk_tokens, chunks_max, s);
+}
+
+// What the kernels over chunks take: 16-byte loads of the queries, of fp16 and of float32 rows, 8-byte loads of int8 rows.
+bool chunk_kernels_take(const SdpaParams& p) {
+  const int group = p.nkv > 0 ? p.n / p.nkv : 0;
+  const uintptr_t kv = reinterpret_cast<uintptr_t>(p.k) | reinterpret_cast<uintptr_t>(p.v);
+  return group >= 1 && group <= 8 && p.n % p.nkv == 0 && (p.h == 256 || p.h == 128 || p.h == 64) && p.ws != nullptr &&
+         p.ws_bytes >= sdpa_chunk_workspace_bytes(p.b, p.nkv, p.h, p.s_max, p.shared_kv) &&
+         (kv & (p.kv_dtype == kKvI8 ? 7 : 15)) == 0 && (reinterpret_cast<uintptr_t>(p.q) & 15) == 0;
+}
+
+template <int KV, int H, bool QF32>
+cudaError_t launch_fast(const SdpaParams& p, cudaStream_t s) {
+  return p.shared_kv ? launch_rows<KV, H, QF32>(p, s) : launch_chunks<KV, H, QF32>(p, s);
 }
 
 template <int KV, bool QF32>
 cudaError_t launch_kv(const SdpaParams& p, cudaStream_t s) {
-  const int group = p.nkv > 0 ? p.n / p.nkv : 0;
-  const bool rows = p.shared_kv && group >= 1 && group <= 8 && p.n % p.nkv == 0 && p.ws != nullptr &&
-                    p.ws_bytes >= sdpa_workspace_bytes(p.b, p.n, p.nkv, p.h, p.s_max, p.shared_kv);
-  if (p.q_tiled_out && (!rows || !QF32 || (p.h != 256 && p.h != 128 && p.h != 64)))
-    return cudaErrorInvalidValue;  // fused output quantization exists on the fast f32-query path only
-  if (rows && p.h == 256) return launch_rows<KV, 256, QF32>(p, s);
-  if (rows && p.h == 128) return launch_rows<KV, 128, QF32>(p, s);
-  if (rows && p.h == 64) return launch_rows<KV, 64, QF32>(p, s);
+  if (chunk_kernels_take(p)) {
+    if (p.h == 256) return launch_fast<KV, 256, QF32>(p, s);
+    if (p.h == 128) return launch_fast<KV, 128, QF32>(p, s);
+    return launch_fast<KV, 64, QF32>(p, s);
+  }
+  if (p.q_tiled_out) return cudaErrorInvalidValue;  // fused output quantization exists on the fast paths only
   const size_t smem = sizeof(float) * ((size_t)p.h + p.s_max);
   auto kernel = sdpa_decode_generic_kernel<KV, QF32>;
   if (smem > 48 * 1024) {
@@ -1481,8 +1579,11 @@ size_t sdpa_chunk_workspace_bytes(int b, int nkv, int h, int s_max, int shared_k
 size_t sdpa_workspace_bytes(int b, int n, int nkv, int h, int s_max, int shared_kv) {
   (void)n;
   const size_t chunks = sdpa_chunk_workspace_bytes(b, nkv, h, s_max, shared_kv);
-  return shared_kv ? chunks : std::max(chunks, sdpa_split_workspace_bytes(b, nkv, h, s_max));
+  // (records are written 16 bytes at a time: room to start on the next boundary)
+  return 16 + (shared_kv ? chunks : std::max(chunks, sdpa_split_workspace_bytes(b, nkv, h, s_max)));
 }
+
+bool sdpa_runs_generic(const SdpaParams& p) { return !sdpa_split_supported(p) && !chunk_kernels_take(p); }
 
 int& expired_waits() {
   static thread_local int v = 0;
@@ -1492,7 +1593,12 @@ int& expired_waits() {
 cudaError_t launch_sdpa_decode(const SdpaParams& given, cudaStream_t s) {
   SdpaParams p = given;
   p.expired = expired_waits();
-  if (sdpa_split_supported(p)) return launch_sdpa_split(p, s);
+  const size_t skip = (16 - (reinterpret_cast<uintptr_t>(p.ws) & 15)) & 15;
+  if (p.ws && p.ws_bytes >= skip) p.ws = reinterpret_cast<float*>(reinterpret_cast<uintptr_t>(p.ws) + skip), p.ws_bytes -= skip;
+  if (sdpa_split_supported(p)) {
+    const cudaError_t e = launch_sdpa_split(p, s);
+    if (e != cudaErrorNotSupported) return e;
+  }
   const bool qf32 = p.q_dtype == 1;
   switch (p.kv_dtype) {
     case kKvF16: return qf32 ? launch_kv<kKvF16, true>(p, s) : launch_kv<kKvF16, false>(p, s);

@@ -94,7 +94,7 @@ struct Pieces {
   }
 };
 
-// Units of all rows, and of the rows below `b`. Whole warp. (32 bits hold them: a unit is at least 1 KB of cache.)
+// Units of all rows, and of the rows below `b`. Whole warp. (32 bits hold them: see sdpa_split_supported.)
 __device__ __forceinline__ void count_units(const SdpaParams& p, int b, int lane, int* total, int* below) {
   int all = 0, low = 0;
   for (int i = lane; i < p.b; i += 32) {
@@ -938,7 +938,7 @@ cudaError_t launch_split(const SdpaParams& p, cudaStream_t s) {
   using S = Split<KV, H, QF32>;
   const long long rows = (long long)(p.rows_per_kv > 1 ? p.b / p.rows_per_kv : p.b) * p.s_max;
   SplitMaps maps;
-  if (!cache_maps<KV, H>(&maps, 0, p.k, p.nkv, rows) || !cache_maps<KV, H>(&maps, 1, p.v, p.nkv, rows)) return cudaErrorInvalidValue;
+  if (!cache_maps<KV, H>(&maps, 0, p.k, p.nkv, rows) || !cache_maps<KV, H>(&maps, 1, p.v, p.nkv, rows)) return cudaErrorNotSupported;
   const int min_units = split_min_units(), ctas = split_ctas(p.b, p.nkv, p.s_max);
   static bool done[64] = {false};
   constexpr size_t smem = split_smem_bytes<KV, H, QF32>();
@@ -972,7 +972,8 @@ bool sdpa_split_supported(const SdpaParams& p) {
   return group >= 1 && group <= 8 && p.n % p.nkv == 0 && (p.h == 64 || p.h == 128 || p.h == 256) && !p.shared_kv &&
          ((reinterpret_cast<uintptr_t>(p.k) | reinterpret_cast<uintptr_t>(p.v) | reinterpret_cast<uintptr_t>(p.q) |
            reinterpret_cast<uintptr_t>(p.ws)) & 15) == 0 &&
-         p.ws != nullptr && p.ws_bytes >= sdpa_split_workspace_bytes(p.b, p.nkv, p.h, p.s_max);
+         (long long)p.b * p.nkv * ((p.s_max + kUnit - 1) / kUnit) <= INT32_MAX && p.ws != nullptr &&
+         p.ws_bytes >= sdpa_split_workspace_bytes(p.b, p.nkv, p.h, p.s_max);
 }
 
 size_t sdpa_split_workspace_bytes(int b, int nkv, int h, int s_max) {

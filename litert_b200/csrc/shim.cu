@@ -298,6 +298,12 @@ int b200_fc_w4(const float* d_x, int m, int k, const void* d_w4_packed, int n, i
 // which needs no workspace but holds all logits of a head in shared memory).
 static bool sdpa_fast_shape(int n, int nkv, int h) { return n % nkv == 0 && n / nkv <= 8 && (h == 64 || h == 128 || h == 256); }
 
+static int check_fallback(const b200::SdpaParams& p, const char* name) {
+  if (!b200::sdpa_runs_generic(p) || sizeof(float) * ((size_t)p.h + p.s_max) <= 200 * 1024) return B200_OK;
+  return fail(B200_ERR_UNSUPPORTED, "%s: this head layout or alignment runs on the fallback kernel, which holds s_max logits in shared "
+              "memory (s_max + h <= 51200)", name);
+}
+
 size_t b200_sdpa_workspace_bytes(int b, int n, int nkv, int h, int s_max) {
   if (b <= 0 || n <= 0 || nkv <= 0 || h <= 0 || s_max <= 0) return 0;
   return b200::sdpa_workspace_bytes(b, n, nkv, h, s_max);
@@ -316,8 +322,6 @@ int b200_sdpa_decode(const void* d_q, const void* d_k, const void* d_v, const fl
   if (sdpa_fast_shape(n, nkv, h) && (!d_workspace || workspace_bytes < b200::sdpa_workspace_bytes(b, n, nkv, h, s_max)))
     return fail(B200_ERR_INVALID_ARGUMENT, "b200_sdpa_decode: workspace too small (%zu < %zu, see b200_sdpa_workspace_bytes)",
                 workspace_bytes, b200::sdpa_workspace_bytes(b, n, nkv, h, s_max));
-  if (!sdpa_fast_shape(n, nkv, h) && sizeof(float) * ((size_t)h + s_max) > 200 * 1024)
-    return fail(B200_ERR_UNSUPPORTED, "b200_sdpa_decode: this head layout runs on the fallback kernel, which holds s_max logits in shared memory (s_max + h <= 51200)");
   b200::SdpaParams p;
   memset(&p, 0, sizeof(p));
   p.q = d_q; p.k = d_k; p.v = d_v; p.k_scale = d_k_scale; p.v_scale = d_v_scale;
@@ -329,6 +333,7 @@ int b200_sdpa_decode(const void* d_q, const void* d_k, const void* d_v, const fl
   p.logit_cap = logit_cap;
   p.ws = static_cast<float*>(d_workspace);
   p.ws_bytes = workspace_bytes;
+  if (int rc = check_fallback(p, "b200_sdpa_decode")) return rc;
   cudaError_t e = b200::launch_sdpa_decode(p, static_cast<cudaStream_t>(stream));
   return e == cudaSuccess ? B200_OK : cuda_fail(e, "b200_sdpa_decode");
 }
@@ -343,8 +348,6 @@ int b200_sdpa(const void* d_q, const void* d_k, const void* d_v, const float* d_
   if (kv_dtype != B200_DTYPE_F16 && kv_dtype != B200_DTYPE_F32) return fail(B200_ERR_UNSUPPORTED, "b200_sdpa: kv dtype %d", kv_dtype);
   if (sdpa_fast_shape(n, nkv, h) && (!d_workspace || workspace_bytes < b200::sdpa_workspace_bytes(b * t, n, nkv, h, s_max)))
     return fail(B200_ERR_INVALID_ARGUMENT, "b200_sdpa: workspace too small (b200_sdpa_workspace_bytes(b * t, ...))");
-  if (!sdpa_fast_shape(n, nkv, h) && sizeof(float) * ((size_t)h + s_max) > 200 * 1024)
-    return fail(B200_ERR_UNSUPPORTED, "b200_sdpa: this head layout runs on the fallback kernel (s_max + h <= 51200)");
   b200::SdpaParams p;
   memset(&p, 0, sizeof(p));
   p.q = d_q; p.k = d_k; p.v = d_v;
@@ -357,6 +360,7 @@ int b200_sdpa(const void* d_q, const void* d_k, const void* d_v, const float* d_
   p.logit_cap = logit_cap;
   p.ws = static_cast<float*>(d_workspace);
   p.ws_bytes = workspace_bytes;
+  if (int rc = check_fallback(p, "b200_sdpa")) return rc;
   cudaError_t e = b200::launch_sdpa_decode(p, static_cast<cudaStream_t>(stream));
   return e == cudaSuccess ? B200_OK : cuda_fail(e, "b200_sdpa");
 }

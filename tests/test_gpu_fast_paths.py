@@ -236,3 +236,79 @@ def test_sdpa_decode_weights_are_not_rounded_to_fp16(ops, ws, kv, n, nkv, h):
     for i, length in enumerate(lengths):
         want = _attention(q[i, 0], k[i], v[i], int(length), 1.0 / np.sqrt(h), 0.0)
         assert np.linalg.norm(out[i, 0] - want) <= 2.0 ** -15 * np.linalg.norm(want), i
+
+
+def _at_offset(a, nbytes):
+    """The array on the device, `nbytes` behind a 256-byte boundary."""
+    flat = torch.from_numpy(np.ascontiguousarray(a)).cuda().reshape(-1)
+    raw = torch.empty(flat.numel() * flat.element_size() + 256, dtype=torch.uint8, device="cuda")
+    at = raw[nbytes:nbytes + flat.numel() * flat.element_size()].view(flat.dtype).reshape(a.shape)
+    at.copy_(flat.reshape(a.shape))
+    assert at.data_ptr() % 256 == nbytes
+    return at
+
+
+@pytest.mark.parametrize("s_max,b", [(700, 5), (60000, 1)])
+@pytest.mark.parametrize("n,nkv,h", [(8, 1, 256), (6, 2, 128), (4, 4, 64)])
+def test_sdpa_decode_int8_cache_on_an_8_byte_boundary(ops, ws, s_max, b, n, nkv, h):
+    """Copies by the TMA need 16 bytes; a cache on 8 is taken by the kernel that loads rows straight, whatever its
+    length. Also quantized. Bound: fp16 weights, queries and outputs, as for the other decode tests."""
+    rng = np.random.default_rng(h + b)
+    lengths = np.asarray([s_max, 0, 1, 65, 640][:b], np.int32)
+    q = rng.standard_normal((b, 1, n, h)).astype(np.float16)
+    kd = rng.integers(-127, 128, (b, s_max, nkv, h)).astype(np.int8)
+    vd = rng.integers(-127, 128, (b, s_max, nkv, h)).astype(np.int8)
+    ks, vs = (rng.uniform(0.005, 0.02, (b, s_max, nkv)).astype(np.float32) for _ in range(2))
+    k, v = _at_offset(kd, 8), _at_offset(vd, 8)
+    out = ops.sdpa_decode(dev(q), k, v, lengths=dev(lengths), k_scale=dev(ks), v_scale=dev(vs), ws=ws).float().cpu().numpy()
+    rows = ops.sdpa_decode_quantized(dev(q.astype(np.float32)), k, v, dev(lengths), k_scale=dev(ks), v_scale=dev(vs))
+    scale, zp = rows.scales[:b].cpu().numpy(), rows.zero_points[:b].cpu().numpy()
+    quant = (rows.rows().cpu().numpy().astype(np.float64) - zp[:, None]) * scale[:, None]
+    for i, length in enumerate(lengths):
+        want = _attention(q[i, 0].astype(np.float32), kd[i].astype(np.float32) * ks[i][..., None],
+                          vd[i].astype(np.float32) * vs[i][..., None], int(length), 1.0 / np.sqrt(h), 0.0)
+        bound = 5 * 2.0 ** -11 * max(np.max(np.abs(want)), 1e-30)
+        assert np.max(np.abs(out[i, 0] - want)) <= bound, i
+        assert np.max(np.abs(quant[i].reshape(n, h) - want)) <= bound + 0.51 * scale[i], i
+
+
+@pytest.mark.parametrize("kv", ["f16", "i8", "f32"])
+def test_sdpa_decode_workspace_on_a_4_byte_boundary(ops, kv):
+    """The records move up to the next boundary: same bits as with an aligned workspace, nothing written outside."""
+    import ctypes
+
+    from litert_b200 import _lib
+
+    rng = np.random.default_rng(5)
+    b, s_max, n, nkv, h = 3, 3000, 8, 2, 128
+    q = dev(rng.standard_normal((b, 1, n, h)).astype(np.float32))
+    x = [rng.standard_normal((b, s_max, nkv, h)) for _ in range(2)]
+    kw = {}
+    if kv == "i8":
+        kv_t = [dev(np.clip(np.rint(a * 40), -127, 127).astype(np.int8)) for a in x]
+        kw = {a: torch.full((b, s_max, nkv), 0.02, device="cuda") for a in ("k_scale", "v_scale")}
+    else:
+        kv_t = [dev(a.astype(np.float16 if kv == "f16" else np.float32)) for a in x]
+    lib = _lib.load()
+    need = lib.b200_sdpa_workspace_bytes(b, n, nkv, h, s_max)
+    guard = torch.full((need + 512,), 0x5A, dtype=torch.uint8, device="cuda")
+    out = torch.empty_like(q)
+    p = lambda t: None if t is None else ctypes.c_void_p(t.data_ptr())
+    _lib.check(lib.b200_sdpa_decode(p(q), p(kv_t[0]), p(kv_t[1]), p(kw.get("k_scale")), p(kw.get("v_scale")), None, None,
+                                    p(out), b, n, nkv, h, s_max, 2, {"f16": 0, "i8": 1, "f32": 2}[kv], 0.0, 0.0,
+                                    ctypes.c_void_p(guard.data_ptr() + 260), need, None))
+    torch.cuda.synchronize()
+    assert torch.equal(out, ops.sdpa_decode(q, *kv_t, ws=ops.Workspace("cuda"), **kw))
+    g = guard.cpu().numpy()
+    assert (g[:260] == 0x5A).all() and (g[260 + need:] == 0x5A).all()
+
+
+def test_sdpa_decode_says_what_it_does_not_take(ops, ws):
+    """fp16 rows on an 8-byte boundary run on the fallback, which holds all logits in shared memory."""
+    from litert_b200._lib import B200Error
+
+    q = torch.randn((1, 1, 8, 64), device="cuda")
+    mk = lambda s: _at_offset(np.zeros((1, s, 1, 64), np.float16), 8)
+    assert not ops.sdpa_decode(q, mk(300), mk(300), ws=ws).any()
+    with pytest.raises(B200Error, match="alignment"):
+        ops.sdpa_decode(q, mk(60000), mk(60000), ws=ws)
