@@ -201,6 +201,7 @@ bool sdpa_runs_generic(const SdpaParams& p);
 size_t sdpa_chunk_workspace_bytes(int b, int nkv, int h, int s_max, int shared_kv = 0);
 // One query row per sequence (sdpa_split.cu): the ragged decode step.
 bool sdpa_split_supported(const SdpaParams& p);
+bool sdpa_split_faster(const SdpaParams& p);
 cudaError_t launch_sdpa_split(const SdpaParams& p, cudaStream_t s);
 size_t sdpa_split_workspace_bytes(int b, int nkv, int h, int s_max);
 

@@ -424,6 +424,172 @@ __global__ void __launch_bounds__(kWarps * 32) sdpa_decode_kernel(const SdpaPara
   }
 }
 
+// Staged variant of the kernel above for fp16 / int8 caches: the CTA's chunk goes through a ring of
+// shared-memory stages of kRingTokens tokens, every cached row fetched by one bulk asynchronous copy
+// (one row per thread and stage: keys by the lower half of the CTA, values by the upper), so a
+// CTA keeps up to stages x 64 KB in flight without holding registers for it, and the warps read
+// their MMA fragments from shared memory (the loads straight from global memory of the kernel
+// above leave the SMs waiting on the long scoreboard with ~7 warps each). Same chunking, same
+// partial records.
+constexpr int kRingTokens = 64;
+constexpr int kRingStagesMax = 3;
+
+template <int KV, int H>
+struct RingLayout {
+  static constexpr int kRowBytes = H * (KV == kKvI8 ? 1 : 2);
+  static constexpr int kPitch = kRowBytes + 16;  // rows 16 bytes apart in the banks
+  static constexpr int kStageBytes = 2 * kRingTokens * kPitch;
+  static constexpr int kParkBytes = (int)sizeof(float) * kWarps * 8 * (H + 4);
+  static size_t smem_bytes(int stages) {
+    const size_t ring = (size_t)stages * kStageBytes;
+    return (ring > (size_t)kParkBytes ? ring : (size_t)kParkBytes) + 128;
+  }
+};
+
+template <int KV, int H, bool QF32>
+__global__ void __launch_bounds__(kWarps * 32) sdpa_decode_ring_kernel(const SdpaParams p, const int chunk_tokens,
+                                                                       const int chunks_max, const int stages,
+                                                                       const int stage_tokens) {
+  using WA = WarpAttention<KV, H, 1>;
+  using L = RingLayout<KV, H>;
+  constexpr int KSTEPS = WA::KSTEPS;
+  static_assert(kWarps * 32 == 2 * kRingTokens, "one row copy per thread and stage");
+  static_assert(kWarps * 16 == kRingTokens, "one 16-token group per warp and stage");
+  // `stage_tokens` (a multiple of 16, at most kRingTokens) tokens per stage: two stages must fit beside a
+  // second CTA on the SM, so that the copy of the next stage runs under the arithmetic of this one
+  const int stage_bytes = 2 * stage_tokens * L::kPitch;
+  extern __shared__ __align__(128) uint8_t ring_smem[];
+  __shared__ float sm_m[kWarps][8], sm_l[kWarps][8];
+  __shared__ int s_abort;
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(ring_smem);  // [kRingStagesMax], 128 bytes reserved
+  uint8_t* ring = ring_smem + 128;
+  float (*sm_o)[8][H + 4] = reinterpret_cast<float (*)[8][H + 4]>(ring);  // after the loop
+  volatile int* abort_flag = &s_abort;
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (tid == 0) {
+    for (int i = 0; i < kRingStagesMax; ++i) mbar_init(&full_bar[i], 1);
+    s_abort = p.expired;
+    mbar_fence_init();
+  }
+  pdl_enter();
+  __syncthreads();
+  const int b = blockIdx.z, kvh = blockIdx.y, chunk = blockIdx.x;
+  const int len = p.lengths ? max(0, min(p.lengths[b], p.s_max)) : p.s_max;
+  const int c0 = chunk * chunk_tokens;
+  if (c0 >= len) return;  // uniform over the CTA, nothing in flight
+  const int c1 = min(len, c0 + chunk_tokens);
+  const int n_sub = (c1 - c0 + stage_tokens - 1) / stage_tokens;
+  const int g = lane >> 2, t = lane & 3;
+  const int group = p.n / p.nkv;
+  const typename WA::Rows cache = WA::cache_rows(p, b, kvh);
+  // With one kv head the cached rows of consecutive tokens follow one another in memory: a stage is then
+  // ONE bulk copy per operand (32 KB of fp16 rows) instead of one per row, unpadded in shared memory. (128
+  // copies of 512 bytes per stage keep the copy engine busier issuing than moving; the 2- to 4-way bank
+  // conflicts of the unpadded rows cost the fragment loads less than that.)
+  const bool contiguous = cache.stride == (size_t)L::kRowBytes;
+  const int pitch = contiguous ? L::kRowBytes : L::kPitch;
+
+  // stage `s` <- tokens [c0 + j * 64, ...): thread r (< 64) fetches key row r, thread 64 + r value row r
+  auto issue = [&](int j) {
+    const int s = j % stages;
+    const int t0 = c0 + j * stage_tokens;
+    const int rows = min(stage_tokens, c1 - t0);
+    uint8_t* stage = ring + (size_t)s * stage_bytes;
+    if (tid == 0) mbar_arrive_expect_tx(&full_bar[s], (uint32_t)(2 * rows * L::kRowBytes));
+    if (contiguous) {
+      if (tid == 0) {
+        bulk_g2s(stage, cache.k + (size_t)t0 * cache.stride, (uint32_t)(rows * L::kRowBytes), &full_bar[s]);
+        bulk_g2s(stage + (size_t)stage_tokens * L::kPitch, cache.v + (size_t)t0 * cache.stride, (uint32_t)(rows * L::kRowBytes),
+                 &full_bar[s]);
+      }
+      return;
+    }
+    const int r = tid & (kRingTokens - 1);
+    if (r < rows) {
+      const bool is_v = tid >= kRingTokens;
+      const uint8_t* src = (is_v ? cache.v : cache.k) + (size_t)(t0 + r) * cache.stride;
+      bulk_g2s(stage + (size_t)(is_v ? stage_tokens : 0) * L::kPitch + (size_t)r * L::kPitch, src, L::kRowBytes, &full_bar[s]);
+    }
+  };
+  int issued = *abort_flag ? 0 : min(stages, n_sub);
+  for (int j = 0; j < issued; ++j) issue(j);
+
+  // ---- Q fragments (as above) while the first stages land ----
+  uint32_t qf[KSTEPS][4];
+  {
+    const bool head_ok = g < group;
+    const int head = kvh * group + (head_ok ? g : 0);
+#pragma unroll
+    for (int i = 0; i < KSTEPS; ++i) {
+      const int d0 = 8 * (t + 4 * i);
+      if (!head_ok) {
+        qf[i][0] = qf[i][1] = qf[i][2] = qf[i][3] = 0u;
+      } else if constexpr (QF32) {
+        const float* q = static_cast<const float*>(p.q) + ((size_t)b * p.n + head) * H + d0;
+        load8<kKvF32>(q, 0, true, qf[i]);
+      } else {
+        const __half* q = static_cast<const __half*>(p.q) + ((size_t)b * p.n + head) * H + d0;
+        load8<kKvF16>(q, 0, true, qf[i]);
+      }
+    }
+  }
+  WA wa;
+  wa.clear();
+  for (int j = 0; j < n_sub; ++j) {
+    const int s = j % stages;
+    mbar_wait_bounded(&full_bar[s], (uint32_t)(j / stages) & 1u, abort_flag, p.status, kStatusWaitTimeoutFull);
+    const int t0 = c0 + j * stage_tokens;
+    const int t1 = min(c1, t0 + stage_tokens);
+    const int first = t0 + warp * 16;
+    if (first < t1 && !*abort_flag) {
+      typename WA::Rows rows = cache;  // scales stay in global memory
+      const uint8_t* stage = ring + (size_t)s * stage_bytes;
+      rows.k = stage - (ptrdiff_t)t0 * pitch;  // indexed by absolute token
+      rows.v = stage + (size_t)stage_tokens * L::kPitch - (ptrdiff_t)t0 * pitch;
+      rows.stride = pitch;
+      wa.template run<kSrcShared>(p, qf, rows, b, first, kRingTokens, t1, lane, /*fresh=*/false, /*finish=*/false);
+    }
+    __syncthreads();  // every warp is done with stage s
+    if (issued < n_sub && !*abort_flag) {  // (abort_flag cannot change between the barrier above and here)
+      issue(issued);
+      ++issued;
+    }
+  }
+  wa.finish_sums();
+  // after an abort: the latest copies towards each stage may still be in flight
+  const bool lost = __syncthreads_or(*abort_flag) != 0;
+  if (lost)
+    for (int j = max(0, issued - stages); j < issued; ++j)
+      mbar_drain_bounded(&full_bar[j % stages], (uint32_t)(j / stages) & 1u);
+  __syncthreads();
+
+  // ---- merge the warps of this CTA (the parked outputs reuse the ring) ----
+  wa.park(sm_m, sm_l, sm_o, warp, lane);
+  __syncthreads();
+  float* part = p.ws + ((((size_t)b * p.nkv + kvh) * chunks_max + chunk) * 8) * partial_stride(H);
+  for (int idx = tid; idx < group * H; idx += kWarps * 32) {
+    const int head = idx / H, d = idx % H;
+    float mm = -CUDART_INF_F;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) mm = fmaxf(mm, sm_m[w][head]);
+    const float muse = mm == -CUDART_INF_F ? 0.0f : mm;
+    float acc = 0.0f, l = 0.0f;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) {
+      const float f = exp2f(sm_m[w][head] - muse);
+      acc += f * sm_o[w][head][d];
+      l += f * sm_l[w][head];
+    }
+    float* rec = part + (size_t)head * partial_stride(H);
+    rec[d] = acc;
+    if (d == 0) {
+      rec[H] = mm;
+      rec[H + 1] = lost ? kLostRecord : l;
+    }
+  }
+}
+
 // Prompt-pass variant (SdpaParams::shared_kv): the rows of the batch are consecutive tokens of ONE
 // sequence and all read the same cache, row b up to lengths[b]. Here a WARP owns a row: the warps of a
 // CTA walk the same chunk of the cache for kWarps neighbouring rows at nearly the same pace, so the
@@ -1445,6 +1611,35 @@ cudaError_t launch_chunks(const SdpaParams& p, cudaStream_t s) {
   const int chunk_tokens = pick_chunk_tokens(p.b, p.s_max, 0);
   const int chunks_max = (p.s_max + chunk_tokens - 1) / chunk_tokens;
   const dim3 grid(chunks_max, p.nkv, p.b);
+  if constexpr (KV != kKvF32) {
+    if (((reinterpret_cast<uintptr_t>(p.k) | reinterpret_cast<uintptr_t>(p.v)) & 15) == 0 && chunk_tokens % kRingTokens == 0) {
+      using L = RingLayout<KV, H>;
+      // Two CTAs per SM (about 104 KB each), at least two stages per CTA so that the next stage's copy runs
+      // under this stage's arithmetic: with ONE 64-token stage per CTA (three CTAs per SM) every CTA of the
+      // grid loads, computes, loads ... in step with the others, HBM idle half of the time (device-timer
+      // stamps of one CTA, 16 ragged sequences, fp16 rows: 2.0 us copy + 1.8 us arithmetic per stage, strictly
+      // in turn). Rows that do not fit two 64-token stages get shorter stages (fp16 at head size 256: 48).
+      int stage_tokens = kRingTokens;
+      while (stage_tokens > 16 && 2 * (2 * stage_tokens * L::kPitch) > 104 * 1024) stage_tokens -= 16;
+      const int stage_bytes = 2 * stage_tokens * L::kPitch;
+      int stages = std::min(kRingStagesMax, (chunk_tokens + stage_tokens - 1) / stage_tokens);
+      stages = std::min(stages, std::max(1, (104 * 1024) / stage_bytes));
+      const size_t ring_bytes = (size_t)stages * stage_bytes;
+      const size_t smem = (ring_bytes > (size_t)L::kParkBytes ? ring_bytes : (size_t)L::kParkBytes) + 128;
+      auto kernel = sdpa_decode_ring_kernel<KV, H, QF32>;
+      static bool configured[64] = {false};
+      int dev = 0;
+      cudaGetDevice(&dev);
+      if (dev < 0 || dev >= 64) dev = 0;
+      if (!configured[dev]) {
+        cudaError_t ea = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::smem_bytes(kRingStagesMax));
+        if (ea != cudaSuccess) return ea;
+        configured[dev] = true;
+      }
+      const cudaError_t e = launch_chained(kernel, grid, dim3(kWarps * 32), smem, s, p, chunk_tokens, chunks_max, stages, stage_tokens);
+      return e == cudaSuccess ? launch_merge<H, QF32>(p, chunk_tokens, chunks_max, s) : e;
+    }
+  }
   auto kernel = chunk_tokens == 64    ? sdpa_decode_kernel<KV, H, QF32, 1>
                 : chunk_tokens == 128 ? sdpa_decode_kernel<KV, H, QF32, 2>
                                       : sdpa_decode_kernel<KV, H, QF32, 4>;
@@ -1595,7 +1790,7 @@ cudaError_t launch_sdpa_decode(const SdpaParams& given, cudaStream_t s) {
   p.expired = expired_waits();
   const size_t skip = (16 - (reinterpret_cast<uintptr_t>(p.ws) & 15)) & 15;
   if (p.ws && p.ws_bytes >= skip) p.ws = reinterpret_cast<float*>(reinterpret_cast<uintptr_t>(p.ws) + skip), p.ws_bytes -= skip;
-  if (sdpa_split_supported(p)) {
+  if (sdpa_split_supported(p) && (sdpa_split_faster(p) || !chunk_kernels_take(p))) {
     const cudaError_t e = launch_sdpa_split(p, s);
     if (e != cudaErrorNotSupported) return e;
   }

@@ -866,18 +866,19 @@ __global__ void __launch_bounds__(kMergeQuantThreads, 2) sdpa_split_merge_quant_
   if (lost && threadIdx.x == 0) p.out_scales[b] = __int_as_float(0x7fffffff);  // (integers hold no NaN; their scale does)
 }
 
-// Shortest piece worth a CTA of its own.
-int split_min_units() {
-  static const int v = [] {
-    const char* e = tuning_env("B200_SDPA_MIN_UNITS");  // measurement knob
-    return e && atoi(e) > 0 ? atoi(e) : 4;
-  }();
-  return v;
+// Shortest piece worth a CTA of its own: one unit where no sequence can leave more than 64 records, the merge's single
+// round trip; longer pieces for longer caches. (Four units whatever the cache made one CTA walk through several short
+// sequences in turn: 16 ragged sequences of up to 64 tokens, 8 heads x 256, fp16 8.8 us, one unit 6.9.)
+int split_min_units(int s_max) {
+  if (const char* e = tuning_env("B200_SDPA_MIN_UNITS")) {  // measurement knob
+    if (atoi(e) > 0) return atoi(e);
+  }
+  return s_max <= 64 * kUnit ? 1 : s_max <= 128 * kUnit ? 2 : 4;
 }
 // CTAs of a launch: one per SM, fewer when even full caches give no piece for some.
 int split_ctas(int b, int nkv, int s_max) {
   const long long most = (long long)b * nkv * ((s_max + kUnit - 1) / kUnit);
-  const long long n = (most + split_min_units() - 1) / split_min_units();
+  const long long n = (most + split_min_units(s_max) - 1) / split_min_units(s_max);
   const int sms = device_sm_count();
   return n < sms ? (int)n : sms;
 }
@@ -939,7 +940,7 @@ cudaError_t launch_split(const SdpaParams& p, cudaStream_t s) {
   const long long rows = (long long)(p.rows_per_kv > 1 ? p.b / p.rows_per_kv : p.b) * p.s_max;
   SplitMaps maps;
   if (!cache_maps<KV, H>(&maps, 0, p.k, p.nkv, rows) || !cache_maps<KV, H>(&maps, 1, p.v, p.nkv, rows)) return cudaErrorNotSupported;
-  const int min_units = split_min_units(), ctas = split_ctas(p.b, p.nkv, p.s_max);
+  const int min_units = split_min_units(p.s_max), ctas = split_ctas(p.b, p.nkv, p.s_max);
   static bool done[64] = {false};
   constexpr size_t smem = split_smem_bytes<KV, H, QF32>();
   cudaError_t e = allow_smem(sdpa_split_kernel<KV, H, QF32>, smem, done);
@@ -974,6 +975,23 @@ bool sdpa_split_supported(const SdpaParams& p) {
            reinterpret_cast<uintptr_t>(p.ws)) & 15) == 0 &&
          (long long)p.b * p.nkv * ((p.s_max + kUnit - 1) / kUnit) <= INT32_MAX && p.ws != nullptr &&
          p.ws_bytes >= sdpa_split_workspace_bytes(p.b, p.nkv, p.h, p.s_max);
+}
+
+// Where the split kernel is the faster one: its chain of barriers and hand-offs costs more than a chunk's loop until there
+// are bytes to wait for, and many pairs of few tokens make a CTA walk through several of them in turn. Over 873 launches
+// of 1 to 16 ragged sequences of up to 8192 tokens, six head layouts, replayed, against the kernels over chunks: 0.89 of
+// their time on average by this rule, 1.0 if everything is split. 16 sequences of up to 512 tokens, 8 heads x 64 on 8 KV
+// heads, int8: 9.0 us over chunks, 13.7 split; of up to 4096 tokens, 8 heads x 256, fp16: 15.6 and 11.3; 300 query tokens
+// over 300, 8 heads x 128, fp16: 22.8 and 33.4. The fused quantization is faster split at every size. (The kernels over
+// chunks keep a weight as one fp16 operand: 2.45e-4 against 64 bits for fp16 rows, 2.1e-4 here.)
+bool sdpa_split_faster(const SdpaParams& p) {
+  if (const char* e = tuning_env("B200_SDPA_SPLIT")) return e[0] != '0';  // measurement knob
+  if (p.q_tiled_out) return true;
+  const long long pairs = (long long)p.b * p.nkv, rows = pairs * p.s_max;
+  const bool long_enough = pairs <= 64 || p.s_max > (p.h == 256 ? 256 : 512);
+  if (p.kv_dtype == kKvF32) return p.h == 64 ? rows > 16384 && pairs <= 256 : long_enough;  // (chunks without staging)
+  if (p.kv_dtype == kKvF16) return p.h == 256 ? long_enough : p.h == 128 ? rows > 8192 && p.s_max > 512 : p.s_max > 2048;
+  return p.s_max > 2048 && rows > 8192 && (p.h > 64 || pairs < 64);
 }
 
 size_t sdpa_split_workspace_bytes(int b, int nkv, int h, int s_max) {

@@ -195,10 +195,10 @@ def _decode_case(rng, lengths, s_max, n, nkv, h):
 @pytest.mark.parametrize("n,nkv,h", [(8, 1, 256), (6, 2, 128), (4, 4, 64)])
 def test_sdpa_decode_int8_value_scales_of_any_size(ops, ws, scales, n, nkv, h):
     """Softmax weights times value scales are fp16 operands: scales far below and above what fp16 holds, and such that
-    change along the cache, cost no more than those near one. Bound: an fp16 rounding (2^-11) of each weight, and half
+    change along the cache, cost no more than those near one (caches over 2048 tokens: the split kernel). Bound: an fp16 rounding (2^-11) of each weight, and half
     the smallest fp16 step (2^-25) of the largest scale, which is counted in units of at most twice itself."""
     rng = np.random.default_rng(h)
-    s_max, lengths = 1500, np.asarray([1500, 0, 700, 33, 1], np.int32)
+    s_max, lengths = 2100, np.asarray([2100, 0, 700, 33, 1], np.int32)
     b = len(lengths)
     q, k8, ks = _decode_case(rng, lengths, s_max, n, nkv, h)
     v8 = rng.integers(-127, 128, (b, s_max, nkv, h)).astype(np.int8)
@@ -222,11 +222,11 @@ def test_sdpa_decode_int8_value_scales_of_any_size(ops, ws, scales, n, nkv, h):
 @pytest.mark.parametrize("kv", ["f16", "f32"])
 @pytest.mark.parametrize("n,nkv,h", [(8, 1, 256), (6, 2, 128), (4, 4, 64)])
 def test_sdpa_decode_weights_are_not_rounded_to_fp16(ops, ws, kv, n, nkv, h):
-    """float16 and float32 rows: a weight is the sum of two fp16 operands (2^-22 of it is lost), so that with operands
+    """float16 and float32 rows in the split kernel: a weight is the sum of two fp16 operands (2^-22 of it is lost), so that with operands
     fp16 holds and float32 outputs only float32 arithmetic is left: 2h products per logit of a few units at 2^-23
     each, taken as 2^-15 of the output. A single fp16 weight is 2^-12 off, 1.8e-4 here."""
     rng = np.random.default_rng(h)
-    s_max, lengths = 900, np.asarray([900, 64, 333], np.int32)
+    s_max, lengths = 2100, np.asarray([2100, 64, 333], np.int32)
     b = len(lengths)
     half = lambda a: a.astype(np.float16).astype(np.float32)
     q = half(rng.standard_normal((b, 1, n, h)))
@@ -312,3 +312,32 @@ def test_sdpa_decode_says_what_it_does_not_take(ops, ws):
     assert not ops.sdpa_decode(q, mk(300), mk(300), ws=ws).any()
     with pytest.raises(B200Error, match="alignment"):
         ops.sdpa_decode(q, mk(60000), mk(60000), ws=ws)
+
+
+@pytest.mark.parametrize("kv", ["f16", "i8", "f32"])
+@pytest.mark.parametrize("b,n,nkv,h,s_max", [(1, 8, 1, 128, 8192), (1, 8, 1, 128, 8193), (2, 8, 8, 64, 1024),
+                                             (2, 8, 8, 64, 1025), (1, 8, 4, 64, 2048), (1, 8, 4, 64, 2049),
+                                             (3, 8, 1, 256, 1023), (3, 8, 1, 256, 1024), (3, 8, 1, 256, 1025),
+                                             (9, 8, 8, 64, 2100), (70, 4, 1, 128, 40), (64, 4, 1, 256, 256), (65, 4, 1, 256, 256),
+                                             (65, 4, 1, 256, 257), (33, 4, 2, 128, 512), (33, 4, 2, 128, 513)])
+def test_sdpa_decode_on_both_sides_of_its_rules(ops, ws, kv, b, n, nkv, h, s_max):
+    """Sizes next to those where another kernel, or another shortest piece, is taken, lengths from nothing to all of the
+    cache. Bound: as for the kernels' other tests, five roundings of 2^-11."""
+    rng = np.random.default_rng(b * s_max)
+    lengths = rng.integers(0, s_max + 1, b).astype(np.int32)
+    lengths[0] = s_max
+    q = rng.standard_normal((b, 1, n, h)).astype(np.float32 if kv == "f32" else np.float16)
+    k, v = (rng.standard_normal((b, s_max, nkv, h)).astype(np.float32) for _ in range(2))
+    kw = {}
+    if kv == "i8":
+        kd, ks = workloads.quantize_kv_per_token(k)
+        vd, vs = workloads.quantize_kv_per_token(v)
+        k, v = kd.astype(np.float32) * ks[..., None], vd.astype(np.float32) * vs[..., None]
+        kw = dict(k_scale=dev(ks), v_scale=dev(vs))
+    else:
+        kd, vd = (a.astype(np.float16 if kv == "f16" else np.float32) for a in (k, v))
+        k, v = kd.astype(np.float32), vd.astype(np.float32)
+    out = ops.sdpa_decode(dev(q), dev(kd), dev(vd), lengths=dev(lengths), ws=ws, **kw).float().cpu().numpy()
+    for i, length in enumerate(lengths):
+        want = _attention(q[i, 0].astype(np.float32), k[i], v[i], int(length), 1.0 / np.sqrt(h), 0.0)
+        assert np.max(np.abs(out[i, 0] - want)) <= 5 * 2.0 ** -11 * max(np.max(np.abs(want)), 1e-30), (i, length)

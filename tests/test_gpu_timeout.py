@@ -137,16 +137,17 @@ def _attention_inputs(kv, b, s, n, nkv, h):
     return q, k, v, kw
 
 
+@pytest.mark.parametrize("s", [1000, 2100])
 @pytest.mark.parametrize("kv", ["f16", "i8", "f32"])
 @pytest.mark.parametrize("n,nkv,h", [(8, 1, 256), (6, 2, 128), (4, 4, 64)])
-def test_attention_whose_waits_run_out_ends_and_the_next_call_is_right(expire_waits, kv, n, nkv, h):
+def test_attention_whose_waits_run_out_ends_and_the_next_call_is_right(expire_waits, kv, n, nkv, h, s):
     """The kernels' loops go on after a wait that ran out, without another copy (a barrier armed twice in a phase has no
     defined state), and end; what runs next is not affected. The result is NaN where there was anything to attend to:
     these entry points have no status word to look at."""
     from litert_b200 import ops
 
-    q, k, v, kw = _attention_inputs(kv, 3, 1000, n, nkv, h)
-    lengths = torch.tensor([1000, 0, 333], dtype=torch.int32, device="cuda")
+    q, k, v, kw = _attention_inputs(kv, 3, s, n, nkv, h)
+    lengths = torch.tensor([s, 0, 333], dtype=torch.int32, device="cuda")
     rows = torch.arange(1, 71, dtype=torch.int32, device="cuda")
     ws = ops.Workspace("cuda")
     one = lambda t: t[0]
@@ -161,7 +162,8 @@ def test_attention_whose_waits_run_out_ends_and_the_next_call_is_right(expire_wa
         torch.cuda.synchronize()
         assert time.perf_counter() - t0 < 1.0
         expire_waits(0)
-        if kv != "f32" or call is calls[0]:  # (float32 rows of a prompt are loaded without a wait)
+        # (float32 rows of a prompt, and of short caches of head size 64, are loaded without a wait)
+        if kv != "f32" or (call is calls[0] and (h > 64 or s > 2048)):
             attended = want.abs().amax(-1) > 0
             assert torch.isnan(got[attended]).all() and not got[~attended].any()
         assert torch.equal(call(), want)
