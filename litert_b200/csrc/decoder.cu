@@ -582,9 +582,9 @@ int ensure_prefill_bufs(b200_decoder* d) {
 // Enqueues the layers over `rows` consecutive prompt tokens of sequence `seq` (tokens and positions
 // already in the prompt scratch). Every projection is one GEMM over all the rows; the rows' keys and
 // values are appended first, then row t attends over the cache up to its own position, which is the
-// causal mask. With `pick`, the last row goes through the final norm, the LM head and the arg-max,
+// causal mask; `end` is the last row's. With `pick`, the last row goes through the final norm, the LM head and the arg-max,
 // whose token lands in next_tokens[seq].
-int enqueue_prefill_chunk(b200_decoder* d, int seq, int rows, bool pick) {
+int enqueue_prefill_chunk(b200_decoder* d, int seq, int rows, int end, bool pick) {
   const b200_decoder_config& c = d->cfg;
   PrefillBufs& f = *d->pf;
   cudaStream_t s = d->stream;
@@ -619,6 +619,7 @@ int enqueue_prefill_chunk(b200_decoder* d, int seq, int rows, bool pick) {
     sp.k_scale = ks;
     sp.v_scale = vs;
     sp.shared_kv = 1;
+    sp.len_bound = end;
     sp.lengths = f.attn_len.as<int32_t>();
     sp.q_tiled_out = f.q_a.as<int8_t>();
     sp.out_scales = f.sc_a.as<float>();
@@ -1078,7 +1079,7 @@ int b200_decoder_prefill(b200_decoder* d, int seq, const int32_t* h_tokens, int 
     }
     DEC_CUDA(cudaMemcpyAsync(f.tokens.p, f.h_stage, sizeof(int32_t) * rows, cudaMemcpyHostToDevice, d->stream));
     DEC_CUDA(cudaMemcpyAsync(f.positions.p, f.h_stage + f.rows, sizeof(int32_t) * rows, cudaMemcpyHostToDevice, d->stream));
-    rc = enqueue_prefill_chunk(d, seq, rows, done + rows == n_tokens);
+    rc = enqueue_prefill_chunk(d, seq, rows, start + done + rows, done + rows == n_tokens);
     if (rc) return rc;
     done += rows;
     DEC_CUDA(cudaStreamSynchronize(d->stream));  // the staging buffer is reused by the next chunk

@@ -167,6 +167,7 @@ struct SdpaParams {
   // 1: every row of the batch attends over the SAME cache (k / v / scales of one sequence, [s_max, nkv, h]),
   // row b up to lengths[b] tokens: a prompt pass, whose rows are consecutive tokens of one sequence
   int shared_kv;
+  int len_bound;  // no length is larger, where the caller knows better than s_max (0: it does not); chooses kernels only
 };
 // One decode step of a decoder layer's attention in one launch (multi-query attention, at most
 // eight query heads): rotary embedding of q and of the new key, cache append, attention over the

@@ -113,9 +113,13 @@ def test_sdpa_rows_of_any_lengths(ops, kv, n, nkv, h, s_max):
     """Query tokens that share one cache, in no order of their lengths: limits on and next to tiles (64 tokens) and
     chunks (256, 320), empty rows, a last CTA that is not full, and cached values that are not finite behind some rows'
     limits. Bound as for the decode step: five roundings of 2^-11."""
+    _check_rows(ops, kv, n, nkv, h, s_max, 83)
+
+
+def _check_rows(ops, kv, n, nkv, h, s_max, more):
     rng = np.random.default_rng(n * 100 + h)
     marks = [0, 1, 63, 64, 65, 127, 128, 129, 255, 256, 257, 319, 320, 321, 640, 1024, s_max - 1, s_max]
-    lengths = np.asarray([m for m in marks if m <= s_max] + list(rng.integers(1, s_max + 1, 83)), np.int32)
+    lengths = np.asarray([m for m in marks if m <= s_max] + list(rng.integers(1, s_max + 1, more)), np.int32)
     rng.shuffle(lengths)
     rows = len(lengths)
     q = rng.standard_normal((rows, n, h)).astype(np.float16)
@@ -139,6 +143,16 @@ def test_sdpa_rows_of_any_lengths(ops, kv, n, nkv, h, s_max):
             continue
         want = _attention(q[i].astype(np.float32), kf, vf, int(length), kw["scale"], kw["logit_cap"])
         assert np.max(np.abs(out[i] - want)) <= 5 * 2.0 ** -11 * max(np.max(np.abs(want)), 1e-30), (i, length)
+
+
+@pytest.mark.parametrize("kv", ["f16", "i8"])
+@pytest.mark.parametrize("n,nkv,h,s_max", [(8, 1, 256, 1100), (7, 1, 128, 700), (6, 2, 64, 330), (4, 4, 256, 164)])
+@pytest.mark.parametrize("above", [0, 1])
+def test_sdpa_rows_on_both_sides_of_their_rule(ops, kv, n, nkv, h, s_max, above):
+    """More than 262144 (row, cached token, KV head) triples run 64 (row, head) pairs to a CTA, others a warp per row:
+    the lengths and values of the test above, one row fewer and one more."""
+    marks = sum(m <= s_max for m in [0, 1, 63, 64, 65, 127, 128, 129, 255, 256, 257, 319, 320, 321, 640, 1024, s_max - 1, s_max])
+    _check_rows(ops, kv, n, nkv, h, s_max, 262144 // (s_max * nkv) + above - marks)
 
 
 @pytest.mark.parametrize("d", [4, 1000, 1024, 1028, 2048, 2052, 4096])
