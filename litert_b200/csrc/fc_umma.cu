@@ -1192,6 +1192,16 @@ __global__ void __launch_bounds__(PrefillLayout<NB>::kThreads, 1) fc_prefill_ker
   if (warp == 1) tmem_dealloc(tmem_base, L::kTmemCols);
 }
 
+// Ranges that the reduction of `tiles` (n tile, pass) pairs is cut into: few tiles and a long reduction are cut so that
+// most SMs get a unit (at least 16 k tiles per range, one scratch slot each).
+int prefill_ksplit(int tiles, int k_tiles) {
+  const int sms = device_sm_count();
+  if (tiles * 2 > sms || k_tiles < 32) return 1;
+  int ks = std::min(sms / tiles, k_tiles / 16);
+  while (ks > 1 && tiles * ks > kZeroWsSlots) --ks;
+  return ks < 1 ? 1 : ks;
+}
+
 template <int EPI, int NB>
 cudaError_t launch_prefill(const FcParams& p, cudaStream_t s) {
   using L = PrefillLayout<NB>;
@@ -1205,17 +1215,9 @@ cudaError_t launch_prefill(const FcParams& p, cudaStream_t s) {
     if (e != cudaSuccess) return e;
     configured[dev] = true;
   }
-  const int passes = (p.m + L::kNB - 1) / L::kNB;
   const int sms = device_sm_count();
-  const int tiles = p.n_tiles * passes;
-  // few tiles, a long reduction: cut it so that most SMs get a unit (at least 16 k tiles per range)
-  int ksplit = 1;
-  if (tiles * 2 <= sms && p.k_tiles >= 32) {
-    ksplit = sms / tiles;
-    if (ksplit > p.k_tiles / 16) ksplit = p.k_tiles / 16;
-    while (ksplit > 1 && tiles * ksplit > kZeroWsSlots) --ksplit;
-    if (ksplit < 1) ksplit = 1;
-  }
+  const int tiles = p.n_tiles * ((p.m + L::kNB - 1) / L::kNB);
+  int ksplit = prefill_ksplit(tiles, p.k_tiles);
   if (const char* e = tuning_env("B200_FC_KSPLIT")) ksplit = atoi(e) > 0 ? atoi(e) : ksplit;  // measurement knob
   const int units = tiles * ksplit;
   const int ctas = units < sms ? units : sms;
@@ -1401,38 +1403,45 @@ cudaError_t try_cluster(const FcParams& p, int nb, cudaStream_t s) {
   }
 }
 
-// Rows per pass of the persistent kernel (64, 128 or 256), by what the launch then costs: waves of (n tile, pass)
-// units, each of which streams k_tiles x (16 KiB of weights + 128 bytes per row) through its SM at the rate L2 gives an
-// SM when all of them pull (80 KB/us; 110 when less than half do) and then stores its outputs. Small passes fill the
-// SMs when there are few n tiles, large ones read the weights fewer times. (Measured at 256 rows per pass whatever the
-// shape: 300 rows of n = 2048, k = 2048 11.8 us, of n = 7360, k = 1536 10.6.)
+// Rows per pass of the persistent kernel (64, 128 or 256), by what the launch then costs, in microseconds: rounds of
+// units over the SMs, each with its epilogue and a k tile every 0.26 us (0.31 at 256 rows; 0.10 while L2 serves few SMs),
+// and the merge of a cut reduction through memory. A k tile costs nearly the same whatever its rows, so the number of
+// rounds decides. Fitted to 2380 launches (1 to 1024 rows, n 128 to 14336, k 128 to 16384), 5 % of error on average; 256
+// rows stay unless another size promises 5 %, or 25 % where its reduction is cut (the merge is what the fit knows least).
+// Against 256 rows for everything over 128: 0.84 of the time on average, 2 shapes longer by 4 %.
 int plan_rows_per_pass(const FcParams& p) {
   const int sms = device_sm_count();
   int best = 256;
   double best_us = 1e30;
   for (int nb = 256; nb >= 64; nb /= 2) {
     if (p.m_alloc % nb != 0) continue;
-    const int units = p.n_tiles * ((p.m + nb - 1) / nb);
-    int waves = (units + sms - 1) / sms;
-    double kt = p.k_tiles;
-    if (nb == 256 && units * 2 <= sms && p.k_tiles >= 32) {  // launch_prefill cuts the reduction then
-      const int ks = std::min(sms / units, p.k_tiles / 16);
-      if (ks > 1) kt = kt / ks + 16;  // (the merge through memory costs as much as some k tiles)
-    }
-    const double rate = units * 2 < sms ? 110.0 : 80.0;
-    const double us = waves * (kt * (16.0 + nb / 8.0) / rate) + nb * 0.013 + 0.5 * waves;
+    const int tiles = p.n_tiles * ((p.m + nb - 1) / nb), ks = prefill_ksplit(tiles, p.k_tiles), units = tiles * ks;
+    const int rounds = (units + sms - 1) / sms, kt = (p.k_tiles + ks - 1) / ks;
+    const double busy = std::min(1.0, (double)units / sms), epilogue = nb == 256 ? 2.2 : nb == 128 ? 1.7 : 1.5;
+    double us = rounds * (epilogue + kt * (0.10 + (nb == 256 ? 0.21 : 0.16) * busy));
+    if (ks > 1) us += 2.0 + 0.5 * ks * nb / 64;
+    if (nb == 256 && p.m > 128) us *= ks > 1 ? 0.75 : 0.95;
     if (us < best_us) best_us = us, best = nb;
   }
   return best;
 }
 
+// Whether more than 64 rows go through the cluster kernel, 64 at a time: few tiles and a reduction long enough to cut.
+// (n = 300, k = 3000, 160 rows 11.1 us against 16.0 persistent; n = 2048, k = 512, 160 rows 12.5 against 7.8.)
+bool cluster_takes_many_rows(const FcParams& p) {
+  const int tiles = p.n_tiles * ((p.m + 63) / 64);
+  return p.k_tiles >= 8 && tiles <= std::min(32, p.k_tiles * 5 / 4 + 3);
+}
+
 template <int EPI>
 cudaError_t launch_all(const FcParams& p, cudaStream_t s) {
   const int nb = umma_rows_per_pass(p.m);
-  // Decode-sized, and anything else with so few tiles that whole ones would leave half the SMs idle: split-K inside
-  // clusters, up to 64 rows per pass.
-  cudaError_t e = try_cluster<EPI>(p, nb <= 64 ? nb : 64, s);
-  if (e != cudaErrorNotSupported) return e;
+  // Decode-sized, and more rows of so few tiles that whole ones would leave most SMs idle: split-K inside clusters, up to
+  // 64 rows per pass.
+  if (nb <= 64 || cluster_takes_many_rows(p)) {
+    const cudaError_t e = try_cluster<EPI>(p, nb <= 64 ? nb : 64, s);
+    if (e != cudaErrorNotSupported) return e;
+  }
   if (p.push_ranks > 1) return cudaErrorInvalidValue;  // only the cluster kernel pushes its outputs to the peers
   if (nb == 16) return launch_umma_one<16, EPI>(p, s);
   if (nb == 32) return launch_umma_one<32, EPI>(p, s);

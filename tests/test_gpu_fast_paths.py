@@ -355,3 +355,36 @@ def test_sdpa_decode_on_both_sides_of_its_rules(ops, ws, kv, b, n, nkv, h, s_max
     for i, length in enumerate(lengths):
         want = _attention(q[i, 0].astype(np.float32), k[i], v[i], int(length), 1.0 / np.sqrt(h), 0.0)
         assert np.max(np.abs(out[i, 0] - want)) <= 5 * 2.0 ** -11 * max(np.max(np.abs(want)), 1e-30), (i, length)
+
+
+_FC_SHAPES = [
+    # cluster kernel: one or two columns and four at a time, one pass and several, partial passes and n tiles
+    (2, 300, 2048), (3, 300, 2048), (17, 4096, 2048), (32, 1000, 3000), (33, 1000, 3000), (64, 2048, 2048), (32, 11000, 512),
+    (300, 200, 1024), (257, 700, 4300), (66, 900, 2048),
+    # persistent kernel, 64 rows per pass: whole reductions and cut ones
+    (66, 1000, 1024), (129, 2000, 700), (128, 6000, 4200), (400, 1300, 4500), (300, 1300, 8300), (90, 2500, 16384),
+    # 128 rows per pass
+    (130, 4097, 1500), (100, 9000, 600), (700, 2000, 300), (150, 2500, 8200), (513, 2100, 5000),
+    # 256 rows per pass
+    (250, 4001, 4096), (200, 8200, 1000), (513, 3001, 2100), (1000, 300, 6000), (512, 1000, 4500)]
+
+
+@pytest.mark.parametrize("m,n,k", _FC_SHAPES)
+def test_fully_connected_by_every_route(ops, ws, oracle, m, n, k):
+    """Shapes that the rules on rows, tiles and reduction length send to each kernel and pass size. Bit-equal to the
+    oracle for the rows next to edges of passes and some others (a row's result does not depend on the other rows)."""
+    rng = np.random.default_rng(m + n + k)
+    rows = sorted({r for e in range(0, m + 64, 64) for r in (e - 1, e) if 0 <= r < m} | {m - 1} | set(rng.integers(0, m, 4).tolist()))
+    w = rng.integers(-127, 128, (n, k)).astype(np.int8)
+    scales = rng.uniform(1e-3, 1e-2, n).astype(np.float32)
+    packed = ops.PackedInt8Weights(dev(w))
+    x = rng.standard_normal((m, k)).astype(np.float32)
+    y = ops.fully_connected_hybrid(dev(x), packed, dev(scales), ws=ws).cpu().numpy()
+    assert np.array_equal(y[rows], oracle.fc_hybrid(x[rows], w, scales))
+    xq = rng.integers(-128, 128, (m, k)).astype(np.int8)
+    bias = rng.integers(-5000, 5001, n).astype(np.int32)
+    out_scale = float(np.float32(0.02 * 5.5e-3 * 74 * np.sqrt(k)))
+    mult, shift = oracle.fc_per_channel_multipliers(0.02, out_scale, scales)
+    yq = ops.fully_connected_int8(dev(xq), packed, dev(bias), 3, -5, dev(mult), dev(shift), ws=ws).cpu().numpy()
+    assert np.array_equal(yq[rows], oracle.fc_int8_per_channel(xq[rows], w, bias, 3, 0.02, scales, out_scale, -5))
+    ws.check_status()
