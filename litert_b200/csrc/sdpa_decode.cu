@@ -1939,6 +1939,7 @@ int& expired_waits() {
 
 cudaError_t launch_sdpa_decode(const SdpaParams& given, cudaStream_t s) {
   SdpaParams p = given;
+  if (p.q_tiled_out && p.q_dtype != 1) return cudaErrorInvalidValue;  // quantized outputs are of float32 queries
   p.expired = expired_waits();
   const size_t skip = (16 - (reinterpret_cast<uintptr_t>(p.ws) & 15)) & 15;
   if (p.ws && p.ws_bytes >= skip) p.ws = reinterpret_cast<float*>(reinterpret_cast<uintptr_t>(p.ws) + skip), p.ws_bytes -= skip;

@@ -388,3 +388,15 @@ def test_fully_connected_by_every_route(ops, ws, oracle, m, n, k):
     yq = ops.fully_connected_int8(dev(xq), packed, dev(bias), 3, -5, dev(mult), dev(shift), ws=ws).cpu().numpy()
     assert np.array_equal(yq[rows], oracle.fc_int8_per_channel(xq[rows], w, bias, 3, 0.02, scales, out_scale, -5))
     ws.check_status()
+
+
+@pytest.mark.parametrize("kv", [np.float16, np.float32])
+def test_quantized_attention_takes_float32_queries_only(ops, kv):
+    from litert_b200._lib import B200Error
+
+    q = torch.randn((2, 1, 8, 128), device="cuda")
+    k = dev(np.zeros((2, 100, 1, 128), kv))
+    lengths = torch.tensor([100, 7], dtype=torch.int32, device="cuda")
+    assert not ops.sdpa_decode_quantized(q, k, k, lengths).rows().any()
+    with pytest.raises(B200Error):
+        ops.sdpa_decode_quantized(q.half(), k, k, lengths)
