@@ -1,10 +1,12 @@
 """ctypes binding of the C ABI (include/litert_b200.h). Fails loudly when the library is missing."""
 import ctypes
+import importlib.util
 import os
+import sys
+import warnings
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "lib", "liblitert_b200.so")
-HOST_OPS_PATH = os.path.join(_HERE, "lib", "_host_ops.so")
 
 _vp = ctypes.c_void_p
 _i = ctypes.c_int
@@ -134,20 +136,37 @@ def load():
     return _lib
 
 
-class _Missing:
-    def __getattr__(self, name):
-        raise B200Error(f"{HOST_OPS_PATH} is missing: build it with `python -m litert_b200.build`")
+def host_ops_path():
+    """The extension of the small calls: one file per interpreter and torch, since it is compiled against both."""
+    import torch
+
+    return os.path.join(_HERE, "lib", f"_host_ops.{sys.implementation.cache_tag}-torch{torch.__version__}.so")
+
+
+class _GeneralPath:
+    """Stands in for the extension: no call is its plain case."""
+
+    @staticmethod
+    def fc_int8(*_):
+        return None
+
+    fc_hybrid = fc_w4 = sdpa_decode = fc_int8
 
 
 def host_ops():
-    """The native form of the small calls (csrc/host_ops.cc); a call raises where it is not built."""
-    if not os.path.exists(HOST_OPS_PATH):
-        return _Missing()
-    import importlib.util
-    load()
-    spec = importlib.util.spec_from_file_location("_host_ops", HOST_OPS_PATH)
-    module = importlib.util.module_from_spec(spec)
-    spec.loader.exec_module(module)
+    """The native form of the small calls (csrc/host_ops.cc). Without it every call takes the general path through
+    ctypes: the same kernels and results, some microseconds more on the host."""
+    path = host_ops_path()
+    if not os.path.exists(path) or not os.path.exists(LIB_PATH):
+        return _GeneralPath
+    try:
+        load()
+        spec = importlib.util.spec_from_file_location("_host_ops", path)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+    except (ImportError, OSError) as e:
+        warnings.warn(f"{path} does not load ({e}): small calls go through ctypes; rebuild with `python -m litert_b200.build`")
+        return _GeneralPath
     return module
 
 

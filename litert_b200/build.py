@@ -58,16 +58,24 @@ def build_kernels(force=False, verbose=False):
 
 
 def build_host_ops(force=False):
-    """The CPython extension of the small calls (csrc/host_ops.cc), over the kernels' library and torch's C++ API."""
+    """The CPython extension of the small calls (csrc/host_ops.cc), over the kernels' library and torch's C++ API, for this
+    interpreter and this torch. None without torch: the calls then go through ctypes."""
+    import glob
     import sysconfig
 
-    import torch
+    try:
+        import torch
+    except ImportError:
+        return None
+    from ._lib import host_ops_path
 
     kernels = build_kernels()
-    out = os.path.join(LIB, "_host_ops.so")
+    out = host_ops_path()
     src = os.path.join(CSRC, "host_ops.cc")
     if not force and not _newer(out, [src, os.path.join(os.path.dirname(HERE), "include", "litert_b200.h")]):
         return out
+    for stale in glob.glob(os.path.join(glob.escape(LIB), "_host_ops*.so")):  # of another torch
+        os.remove(stale)
     root = os.path.dirname(torch.__file__)
     inc = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
            sysconfig.get_paths()["include"], os.path.join(os.path.dirname(os.path.dirname(NVCC)), "include")]
@@ -80,7 +88,7 @@ def build_host_ops(force=False):
 
 
 def build_all(force=False, verbose=False):
-    paths = [build_kernels(force, verbose), build_host_ops(force)]
+    paths = [p for p in (build_kernels(force, verbose), build_host_ops(force)) if p]
     try:
         from . import build_delegate
     except ImportError:

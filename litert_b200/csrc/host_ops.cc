@@ -119,7 +119,7 @@ struct Fc {
   }
 };
 
-// (x, weights, bias, input_offset, filter_offset, output_offset, multipliers, shifts, act_min, act_max, ws, out)
+// (x, weights, bias, input_zero_point, filter_zero_point, output_zero_point, multipliers, shifts, act_min, act_max, ws, out)
 PyObject* fc_int8(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   if (nargs != 12 || a[10] == Py_None) Py_RETURN_NONE;
   try {
@@ -128,17 +128,17 @@ PyObject* fc_int8(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     if (!f.ok) Py_RETURN_NONE;
     Attr rs_o(a[1], s_row_sums);
     In rs(rs_o.o, at::kInt), bias(a[2], at::kInt, true), mult(a[6], at::kInt), shift(a[7], at::kInt);
-    int in_off, f_off, out_off, lo, hi;
-    if (!rs.ok || !bias.ok || !mult.ok || !shift.ok || !as_int(a[3], &in_off) || !as_int(a[4], &f_off) ||
-        !as_int(a[5], &out_off) || !as_int(a[8], &lo) || !as_int(a[9], &hi))
+    int in_zp, f_zp, out_zp, lo, hi;
+    if (!rs.ok || !bias.ok || !mult.ok || !shift.ok || !as_int(a[3], &in_zp) || !as_int(a[4], &f_zp) ||
+        !as_int(a[5], &out_zp) || !as_int(a[8], &lo) || !as_int(a[9], &hi) || in_zp == INT32_MIN || f_zp == INT32_MIN)
       Py_RETURN_NONE;
     at::Tensor y = result(a[11], std::array<int64_t, 2>{f.m, f.n}, at::kChar, *x.t);
     if (!y.defined()) Py_RETURN_NONE;
     void* s = stream();
     int rc;
     Py_BEGIN_ALLOW_THREADS
-    rc = b200_fc_int8(x.ptr<int8_t>(), f.m, f.k, f.packed.ptr<void>(), f.n, rs.ptr<int32_t>(), bias.ptr<int32_t>(), in_off,
-                      f_off, out_off, mult.ptr<int32_t>(), shift.ptr<int32_t>(), mult.t->numel() > 1 ? 1 : 0, lo, hi,
+    rc = b200_fc_int8(x.ptr<int8_t>(), f.m, f.k, f.packed.ptr<void>(), f.n, rs.ptr<int32_t>(), bias.ptr<int32_t>(), -in_zp,
+                      -f_zp, out_zp, mult.ptr<int32_t>(), shift.ptr<int32_t>(), mult.t->numel() > 1 ? 1 : 0, lo, hi,
                       static_cast<int8_t*>(y.data_ptr()), f.zero.ptr<void>(), f.scratch.ptr<void>(),
                       (size_t)f.scratch.t->numel(), s);
     Py_END_ALLOW_THREADS
@@ -208,7 +208,7 @@ PyObject* fc_w4(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
 
 // (q, k, v, lengths, mask, scale, logit_cap, k_scale, v_scale, ws)
 PyObject* sdpa_decode(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
-  if (nargs != 10 || a[9] == Py_None) Py_RETURN_NONE;
+  if (nargs != 10 || a[9] == Py_None || a[6] == Py_None) Py_RETURN_NONE;
   try {
     if (!THPVariable_CheckExact(a[0]) || !THPVariable_CheckExact(a[1])) Py_RETURN_NONE;
     const at::ScalarType qt = THPVariable_Unpack(a[0]).scalar_type(), kt = THPVariable_Unpack(a[1]).scalar_type();

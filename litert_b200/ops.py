@@ -114,7 +114,7 @@ def fully_connected_int8(x, weights, bias, input_zero_point, output_zero_point, 
                          act_max=127, filter_zero_point=0, ws=None, out=None):
     """Full-integer FULLY_CONNECTED (tflite/kernels/fully_connected.cc:1383-1421 per channel, 1255-1285 per
     tensor). x int8 [..., k]; multipliers/shifts int32 tensors with n entries (per channel) or one."""
-    y = _host.fc_int8(x, weights, bias, -input_zero_point, -filter_zero_point, output_zero_point, multipliers, shifts,
+    y = _host.fc_int8(x, weights, bias, input_zero_point, filter_zero_point, output_zero_point, multipliers, shifts,
                       act_min, act_max, ws, out)
     if y is not None:
         return y
