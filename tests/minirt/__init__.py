@@ -22,12 +22,20 @@ _NP = {F32: np.float32, I32: np.int32, U8: np.uint8, I8: np.int8, F16: np.float1
 OP_ADD, OP_FULLY_CONNECTED, OP_SOFTMAX = 0, 9, 25
 
 
+def _headers():
+    return os.path.exists(os.path.join(LITERT_ROOT, "tflite", "core", "c", "common.h"))
+
+
+def available():
+    """Whether the runtime is built or can be."""
+    return os.path.exists(LIB) or _headers()
+
+
 def build():
     from litert_b200 import build_delegate
 
     src = os.path.join(HERE, "minirt.cc")
-    have = os.path.exists(os.path.join(LITERT_ROOT, "tflite", "core", "c", "common.h"))
-    if not have:
+    if not _headers():
         if os.path.exists(LIB):
             return LIB
         raise RuntimeError("libminirt.so is missing and the LiteRT headers are not available to build it")

@@ -12,6 +12,13 @@ from tests.minirt import F16, F32, I4, I8, I32, OP_SOFTMAX
 pytestmark = pytest.mark.gpu
 
 
+@pytest.fixture(autouse=True)
+def _built(plugin_path):
+    """Skips where the plugin (see plugin_path) or the mini runtime is not built and the LiteRT headers are absent."""
+    if not minirt.available():
+        pytest.skip("mini runtime not built and LiteRT headers absent")
+
+
 @pytest.fixture()
 def rt():
     m = minirt.MiniRuntime()
