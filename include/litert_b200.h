@@ -199,9 +199,9 @@ B200_API int b200_sdpa_rows(const void* d_q, const void* d_k, const void* d_v, c
  * else's fixed memory budget, code being recorded for replay) and therefore
  * cannot supply the workspace b200_sdpa_decode asks for. Same arguments and
  * results as b200_sdpa_decode, minus the workspace: the split-K partials go to
- * a built-in device array of b200_sdpa_static_workspace_limit() bytes (8 MiB,
- * held by every GPU that loads the library until exit). Shapes that need more
- * are rejected with B200_ERR_UNSUPPORTED. The first call on a device looks up
+ * a built-in device array (10 MiB, held by every GPU that loads the library
+ * until exit). Shapes whose chunked records need more than
+ * b200_sdpa_static_workspace_limit() bytes (8 MiB) are rejected with B200_ERR_UNSUPPORTED. The first call on a device looks up
  * the array's device address (set-up; make it before any stream capture).
  * Calls share the array: calls that overlap on the GPU race, serialise them.
  * The array is the current device's: make the stream's device current first (a

@@ -58,8 +58,9 @@ struct UmmaShared {
 // kernel of a programmatically chained sequence gets a CTA onto every SM and fills its ring while
 // this kernel's CTAs are still streaming. Measured on B200 on the batch-1 decode step (18 layers +
 // LM head, 1024-token context): one 180 KB CTA per SM 1.100 ms, one 108 KB CTA 1.070 ms, two 72 KB
-// CTAs 0.97-1.00 ms, three 54 KB CTAs 1.022 ms. With more rows per pass the stages are larger and
-// the deep ring of a single CTA per SM does better (batch 32: 1.667 ms against 1.70 ms).
+// CTAs 0.97-1.00 ms, three 54 KB CTAs 1.022 ms. Up to 32 rows two CTAs of 108 KB share an SM as well
+// (decode step of 32 sequences 1.55 -> 1.29 ms with the attention's change); with more rows per pass the
+// stages are larger and a single CTA per SM keeps a deep ring.
 #ifndef B200_UMMA_KB16
 #define B200_UMMA_KB16 72
 #endif
@@ -867,9 +868,9 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) fc_cluster_kernel(const FcPar
 }
 
 // ---- prefill-sized variant ------------------------------------------------------------------------
-// 256 activation rows per pass, whole work units per CTA, persistent CTAs: a unit is (n tile, pass of
-// 256 rows, k range) and a CTA takes units blockIdx.x, blockIdx.x + gridDim.x, ... One 16 KiB weight
-// tile + the 32 KiB activation tile per stage; the two 256-column accumulators alternate, so the
+// NB = 64, 128 or 256 activation rows per pass (plan_rows_per_pass), whole work units per CTA, persistent
+// CTAs: a unit is (n tile, pass, k range) and a CTA takes units blockIdx.x, blockIdx.x + gridDim.x, ... One
+// 16 KiB weight tile + the activation tile of NB x 128 bytes per stage; two NB-column accumulators alternate, so the
 // epilogue of a unit runs under the MMAs of the CTA's next unit. Eight epilogue warps, two per TMEM
 // lane quarter, each pair splitting the unit's activation rows. 4-byte outputs leave straight from
 // the registers (for one activation row a warp holds 32 consecutive output channels: one full
@@ -884,7 +885,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) fc_cluster_kernel(const FcPar
 template <int NB_>
 struct PrefillLayout {
   static constexpr int kNB = NB_;
-  static constexpr int kQBytes = kNB * kTileK8;                      // 32 KiB
+  static constexpr int kQBytes = kNB * kTileK8;
   static constexpr int kStageBytes = kTileBytes + kQBytes;
   static constexpr int kStagesRaw = (NB_ == 256 ? 206 : 194) * 1024 / kStageBytes;
   static constexpr int kStages = kStagesRaw > 8 ? 8 : kStagesRaw;
@@ -1270,7 +1271,7 @@ cudaError_t launch_umma_one(const FcParams& p, cudaStream_t s) {
   return launch_chained(kernel, dim3(ctas), dim3(kUmmaThreads), smem, s, q);
 }
 
-// Largest split of {8, 4, 2} whose clusters all fit on the device at once, 0 when the shape is
+// Largest split of 8 to 2 (12 for a long reduction) whose clusters all fit on the device at once, 0 when the shape is
 // better served by the kernels above (many n tiles, or a single k tile).
 template <int NB, int EPI>
 int plan_cluster_split(const FcParams& p) {

@@ -1,12 +1,13 @@
-// Attention over a key-value cache: the rows of a prompt pass, a decoder layer's whole attention step in one launch,
-// and the fallback for head layouts that nothing else takes (the ragged decode step is in sdpa_split.cu).
+// Attention over a key-value cache: short caches and unaligned ones of a decode step (sdpa_split.cu has the others), the
+// rows of a prompt pass, a decoder layer's whole attention step in one launch, and the fallback for head layouts that
+// nothing else takes.
 //
 // Math (tflite/experimental/genai/sdpa.cc:361-662): for each query head n of
 // batch entry b, out = softmax_s(scale * q.k_s + mask_s) . v_s over the first
 // len[b] cached tokens of kv head n / (N / Nkv).
 //
-// HBM-bound: every K and V row is read exactly once, straight from global
-// memory into MMA fragments (no shared-memory staging, no transposes):
+// What the kernels have in common (WarpAttention; the prompt kernel over (row, head) pairs has its own comment): K and V rows
+// go from memory, or from a ring of shared-memory stages, into MMA fragments without transposes:
 //  * the up-to-8 query heads sharing a kv head form the 8-wide MMA dimension,
 //    16 cached tokens the 16-row one: S^T[token, head] = K[token, :] . Q^T.
 //    K rows are the row-major A operand as they lie in memory; a thread's

@@ -1,4 +1,5 @@
-// Flash-decode for odml.scaled_dot_product_attention, one query row per sequence: ragged lengths, up to eight
+// Flash-decode for odml.scaled_dot_product_attention, one query row per sequence, where there are bytes to wait for
+// (sdpa_split_faster; sdpa_decode.cu has the kernels for short caches): ragged lengths, up to eight
 // query heads per KV head, fp16 / int8 / float32 caches, optional additive mask and logit cap.
 //
 // Math (tflite/experimental/genai/sdpa.cc:361-662): for each query head, out = softmax_s(scale * q.k_s + mask_s) . v_s
